@@ -11,11 +11,13 @@
 // for GPUs" (2022). One upfront kernel counts the histogram of every digit position in a
 // single read of the keys. Then each digit pass, lowest digit first, reads and writes the
 // keys once:
-//   1. a CTA claims the next tile (atomic counter, so every tile it waits on belongs to a
-//      CTA that is already running or done) and loads its keys, warp-striped;
+//   1. a persistent CTA claims the next tile (atomic counter, so every tile it waits on
+//      belongs to a CTA that is already running or done) and loads its keys, warp-striped,
+//      while the tile before it is looked back and written;
 //   2. ranks them stably by the current digit, warp by warp: each warp walks its keys in
-//      index order and, per 32 keys, groups lanes with equal digits (shared lane masks), so
-//      a key's rank is the warp's running count of its digit plus its lower peers;
+//      index order and, per 32 keys, groups lanes with equal digits (eight ballots and
+//      shared lane masks in turn), so a key's rank is the warp's running count of its digit
+//      plus its lower peers;
 //   3. publishes the tile's 256 digit counts at once (state AGG), then finds each digit's
 //      global offset by decoupled look-back over the per-(tile, digit) words of earlier
 //      tiles (one thread per digit) and publishes the inclusive count (state INC); tile 0
@@ -45,49 +47,44 @@ constexpr uint64_t kStInc = uint64_t(2) << kValBits;
 constexpr int kEpochShift = 42;
 constexpr int kLookWindow = 4;  // predecessor words a look-back step loads at once
 
+// Keys per thread ("rows" of 32 keys per warp) of the largest tile, at two 256-thread CTAs per
+// SM. What bounds a pass is neither HBM (a fifth busy) nor one pipe, but the ALU (ballots) and
+// the shared-memory pipe (random digits) at about 70 % each, plus a cost per tile (counts,
+// digit scan, look-back) of some 4,000 cycles: large tiles of few warps win until the keys and
+// their ranks no longer fit the 128 registers. Digit pass measured on B200, 2^26 uint32 keys /
+// 2^25 int64 keys: 512 threads x 24 / 16 rows, one tile per CTA (as it was) 306 / 215 us; 256 x
+// 48 / 32 226 / 169; 256 x 56 / 36 223 / 166; 64 rows 222 / -, 40 rows - / 184 (spills). Three
+// CTAs per SM of 256 x 36 / 24 242 / 190.
 template <typename K> struct RadixShape;
-// Keys per thread and CTAs per SM of each key size; build-time knobs (-D) for sweeps.
-// Measured on 2^26 uint32 keys (digit pass): 16 keys at 3 CTAs/SM 0.327 ms, 16 at 2 0.350,
-// 20 at 2 0.329, 24 at 2 0.315 ms (fewer, larger tiles: fewer look-backs; 64 registers,
-// no spills).
-#ifndef PXB_RADIX_ITEMS32
-#define PXB_RADIX_ITEMS32 24
-#endif
-#ifndef PXB_RADIX_CTAS32
-#define PXB_RADIX_CTAS32 2
-#endif
-// 8-byte keys, 2^26 int64 sort (eight passes) / 122 M-record segmented key-value sort (four):
-// 8 keys at 3 CTAs/SM 3.77 / 4.12 ms, 12 at 2 3.50 / 3.99, 16 at 2 3.42 / 4.05 ms (64
-// registers, no spills; 16 x 8 B is the largest tile two CTAs per SM can stage).
-#ifndef PXB_RADIX_ITEMS64
-#define PXB_RADIX_ITEMS64 16
-#endif
-#ifndef PXB_RADIX_CTAS64
-#define PXB_RADIX_CTAS64 2
-#endif
 template <> struct RadixShape<uint32_t> {
-    static constexpr int BLOCK = 512, ITEMS = PXB_RADIX_ITEMS32, CTAS = PXB_RADIX_CTAS32;
+    static constexpr int BLOCK = 256, ITEMS = 56, CTAS = 2;
 };
 template <> struct RadixShape<uint64_t> {
-    static constexpr int BLOCK = 512, ITEMS = PXB_RADIX_ITEMS64, CTAS = PXB_RADIX_CTAS64;
+    static constexpr int BLOCK = 256, ITEMS = 36, CTAS = 2;
 };
 
-// Each warp may rank its keys as kSubs independent streams (consecutive parts of its keys),
-// each with its own count and mask tables, so the dependency chains overlap. Measured on a
-// 2^26-key pass: one stream at three CTAs per SM (0.338 ms, some registers spilled to fit)
-// beats two streams at two CTAs per SM (0.362 ms) and at three (0.378 ms).
-constexpr int kSubs = 1;
+// Rows per warp of a tile of `keys` keys: a tile is spread over all warps in whole steps of
+// kRowStep rows (the end is padded with the largest key). Steps of four keep the row loop's
+// bounds checks off every row (239 against 252 us per pass with a check per row).
+constexpr int kRowStep = 4;
+template <int BLOCK>
+__host__ __device__ __forceinline__ uint32_t rows_of(uint32_t keys) {
+    return (keys + BLOCK * kRowStep - 1) / (BLOCK * kRowStep) * kRowStep;
+}
 
+// One tile of keys and two [warps][256] tables (counts, lane masks).
 template <typename K>
 constexpr size_t radix_smem() {
     return (size_t)RadixShape<K>::BLOCK * RadixShape<K>::ITEMS * sizeof(K) +
-           (size_t)(RadixShape<K>::BLOCK / 32) * kSubs * kBins * sizeof(uint32_t) +
-           (size_t)RadixShape<K>::BLOCK * RadixShape<K>::ITEMS * sizeof(uint16_t);
+           (size_t)(RadixShape<K>::BLOCK / 32) * kBins * sizeof(uint32_t) * 2;
 }
 
 template <typename K>
 __device__ __forceinline__ uint32_t digit_of(K k, int shift) {
-    return (uint32_t)(k >> shift) & 0xffu;
+    if constexpr (sizeof(K) == 8)  // shift is a multiple of 8 and the same for all threads
+        return __byte_perm((uint32_t)(k >> (shift & 32)), 0u, 0x4440u | ((uint32_t)shift >> 3 & 3u));
+    else
+        return __byte_perm((uint32_t)k, 0u, 0x4440u | ((uint32_t)shift >> 3));
 }
 
 __device__ __forceinline__ uint64_t ld_relaxed_u64(const uint64_t* p) {
@@ -98,9 +95,25 @@ __device__ __forceinline__ uint64_t ld_relaxed_u64(const uint64_t* p) {
 __device__ __forceinline__ void st_relaxed_u64(uint64_t* p, uint64_t v) {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
-// Which 32-bit half of a ranking-table word holds the lane mask of digit d (1 = high).
-__device__ __forceinline__ uint32_t mask_half(uint32_t d) { return (d >> 4) & 1u; }
-
+// Lanes whose 8-bit digit equals this lane's: eight ballots, each inverted where the lane's
+// own bit is clear (a test that sets a predicate, the vote, a predicated NOT and half an AND
+// per bit).
+__device__ __forceinline__ uint32_t ballot_peers(uint32_t d) {
+    uint32_t peers = 0xffffffffu;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        uint32_t m;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "and.b32 %0, %1, %2;\n\t"
+            "setp.ne.u32 p, %0, 0;\n\t"
+            "vote.sync.ballot.b32 %0, p, 0xffffffff;\n\t"
+            "@!p not.b32 %0, %0;\n\t}"
+            : "=r"(m) : "r"(d), "r"(1u << b));
+        peers &= m;
+    }
+    return peers;
+}
 __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
@@ -199,17 +212,17 @@ template <typename K, int XF_IN, int XF_OUT, bool SEG = false>
 __global__ void __launch_bounds__(RadixShape<K>::BLOCK, RadixShape<K>::CTAS)
     k_radix_pass(const K* __restrict__ in_, K* __restrict__ out_, uint64_t n_, int shift,
                  const unsigned long long* __restrict__ hist, uint64_t* status, uint32_t epoch_,
-                 uint64_t tiles, uint32_t* counters, volatile int32_t* err, SegRadix sr) {
+                 uint32_t tiles_, uint32_t tile_rows, uint32_t* counters, volatile int32_t* err,
+                 SegRadix sr) {
     constexpr int BLOCK = RadixShape<K>::BLOCK, ITEMS = RadixShape<K>::ITEMS;
     constexpr int TILE = BLOCK * ITEMS, WARPS = BLOCK / 32;
-    constexpr int TABLES = WARPS * kSubs, STREAM_ITEMS = ITEMS / kSubs;
-    static_assert(BLOCK >= kBins, "one thread per digit");
-    static_assert(ITEMS % kSubs == 0, "whole streams");
+    constexpr int G = kRowStep;
+    static_assert(BLOCK == kBins, "one thread per digit");
+    static_assert(ITEMS % G == 0 && 32 * ITEMS <= 0xffff, "whole steps, two 16-bit ranks per register");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     K* const s_keys = reinterpret_cast<K*>(smem_raw);
+    // [WARPS][kBins]: each warp's running count of every digit, then its offset in the tile
     uint32_t* const s_wh = reinterpret_cast<uint32_t*>(smem_raw + (size_t)TILE * sizeof(K));
-    // each key's rank within its stream, at the key's tile position (kept out of registers)
-    uint16_t* const s_rank = reinterpret_cast<uint16_t*>(s_wh + TABLES * kBins);
     __shared__ uint64_t s_goff[kBins];
     __shared__ uint32_t s_goff32[kBins];
     __shared__ uint64_t s_part64[kBins / 32];
@@ -217,155 +230,182 @@ __global__ void __launch_bounds__(RadixShape<K>::BLOCK, RadixShape<K>::CTAS)
     __shared__ uint32_t s_tile;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) s_tile = atomicAdd(&counters[0], 1u);
-    // offsets of stream s of this warp in the tile, per digit (filled in step 3a): wh + s * kBins
-    uint32_t* const wh = s_wh + warp * kSubs * kBins;
-    // the ranking's tables borrow the key buffer, which is free until step 4a: one 64-bit
-    // word per (stream, digit) holding the stream's running count of the digit and the lane
-    // mask of the current item's peers, so one load reads both. The mask is the low half for
-    // digits with bit 4 clear and the high half otherwise: digit d's word spans banks 2d and
-    // 2d + 1 (mod 32), so the atomic ORs of a warp spread over all 32 banks, not 16.
-    static_assert((size_t)TILE * sizeof(K) >= (size_t)TABLES * kBins * 8, "rank tables fit");
-    uint64_t* const wm = reinterpret_cast<uint64_t*>(s_keys) + warp * kSubs * kBins;
-#pragma unroll
-    for (int i = lane; i < kSubs * kBins; i += 32) wm[i] = 0ull;
-    __syncthreads();
-    const uint64_t tile = s_tile;
-    // plain: tile `tile` of the array; segmented: work item `tile` is tile tk of segment seg
-    const K* in = in_;
-    K* out = out_;
-    uint64_t n = n_, tk = tile, seg = 0;  // tk: tile index within the array / segment
-    uint32_t epoch = epoch_;
-    if constexpr (SEG) {
-        if (tile >= sr.item_start[sr.S]) {  // the grid is an upper bound of the work items
-            if (tid == 0) persistent_exit(counters);
-            return;
-        }
-        seg = sr.item_seg[tile];
-        tk = tile - sr.item_start[seg];
-        n = sr.src.len(seg);
-        if (n < 2) {  // sorted already; such a segment may come without a temporary
-            if (tid == 0) persistent_exit(counters);
-            return;
-        }
-        const uint64_t a = sr.src.in_addr(seg), b = sr.src.aux_addr(seg);
-        in = reinterpret_cast<const K*>(sr.parity ? b : a);
-        out = reinterpret_cast<K*>(sr.parity ? a : b);
-        epoch = *sr.epoch_base + sr.pos;
-    } else if (tile >= tiles) {  // claim counter out of step: touch nothing
-        if (tid == 0) {
-            *err = kErrRadixRange;
-            persistent_exit(counters);
-        }
-        return;
-    }
-    const uint64_t base = tk * TILE;
-    const uint64_t rem = n - base;
-    const uint32_t valid = rem < (uint64_t)TILE ? (uint32_t)rem : (uint32_t)TILE;
-
-    // 1. keys of warp w: tile positions [w * 32 * ITEMS, (w + 1) * 32 * ITEMS), item i of
-    // lane l at w * 32 * ITEMS + 32 i + l, so items walked in order visit keys in index order
-    K k[ITEMS];
-    const uint32_t w0 = (uint32_t)warp * 32 * ITEMS + lane;
-    if (valid == (uint32_t)TILE) {
-#pragma unroll
-        for (int i = 0; i < ITEMS; ++i) k[i] = to_key<K, XF_IN>(__ldcs(in + base + w0 + 32 * i));
-    } else {
-#pragma unroll
-        for (int i = 0; i < ITEMS; ++i) {
-            const uint32_t li = w0 + 32 * i;  // padding: the largest key, digit 255 at the end
-            k[i] = li < valid ? to_key<K, XF_IN>(in[base + li]) : ~K(0);
-        }
-    }
-
-    // 2. stable warp-level ranking by the current digit. Lanes holding the same digit find
-    // each other through a per-stream table of 256 lane masks (shared-memory atomic OR of
-    // the lane's bit into the low half of the digit's word, read back together with the
-    // count in the high half, then the group's highest lane writes count + peers with a
-    // cleared mask); a key's rank is the stream's running count of its digit plus its lower
-    // peers. This keeps the ranking off the SM's narrow branch unit (where match-any issues)
-    // and off the ALU (eight ballots per key cost more than the whole pass), with three
-    // shared-memory accesses per key.
-    static_assert(32 * STREAM_ITEMS <= 0xffff, "ranks fit 16 bits");
-
     const uint32_t lt = lanemask_lt();
-    const uint32_t le = lt | (1u << lane);
-#pragma unroll
-    for (int j = 0; j < STREAM_ITEMS; ++j) {  // item j of every stream
-        uint32_t d[kSubs], peers[kSubs], c[kSubs], ms[kSubs];
-#pragma unroll
-        for (int t = 0; t < kSubs; ++t) {
-            const uint32_t dg = digit_of(k[t * STREAM_ITEMS + j], shift);
-            d[t] = dg + t * kBins;
-            ms[t] = mask_half(dg);
-            atomicOr(reinterpret_cast<uint32_t*>(&wm[d[t]]) + ms[t], 1u << lane);
-        }
-        __syncwarp();
-#pragma unroll
-        for (int t = 0; t < kSubs; ++t) {
-            const uint64_t v = wm[d[t]];
-            peers[t] = (uint32_t)(v >> (32 * ms[t]));
-            c[t] = (uint32_t)(v >> (32 - 32 * ms[t])) + __popc(peers[t] & lt);
-        }
-        __syncwarp();
-#pragma unroll
-        for (int t = 0; t < kSubs; ++t)  // the highest peer: count + peers, mask cleared
-            if ((peers[t] & ~le) == 0) wm[d[t]] = (uint64_t)(c[t] + 1) << (32 - 32 * ms[t]);
-        __syncwarp();
-#pragma unroll
-        for (int t = 0; t < kSubs; ++t) {
-            const int i = t * STREAM_ITEMS + j;
-            s_rank[w0 + 32 * i] = (uint16_t)c[t];
-        }
-    }
+    const uint32_t self = 1u << lane;
+    if (tid == 0) s_tile = atomicAdd(&counters[0], 1u);
+    uint32_t* const wh = s_wh + warp * kBins;
+    uint32_t* const wm = s_wh + (WARPS + warp) * kBins;
+    for (int i = lane; i < kBins; i += 32) wh[i] = wm[i] = 0u;
+    const uint32_t tiles = SEG ? sr.item_start[sr.S] : tiles_;
+    const uint32_t epoch = SEG ? *sr.epoch_base + sr.pos : epoch_;
+    const uint32_t tile_keys = BLOCK * tile_rows;
     __syncthreads();
 
-    // 3a. per digit: counts of the streams -> exclusive over streams (in key order); tile
-    // count; publish AGG. Then the digit's start in the tile is added to every stream's
-    // offset, so step 4a finds a key's slot with one table read.
-    uint32_t cnt = 0;
-    if (tid < kBins) {
-        const uint64_t* const all = reinterpret_cast<const uint64_t*>(s_keys);
-#pragma unroll 8
-        for (int w = 0; w < TABLES; ++w) {
-            const uint32_t c = (uint32_t)(all[w * kBins + tid] >> (32 - 32 * mask_half(tid)));
-            s_wh[w * kBins + tid] = cnt;
-            cnt += c;
+    // plain: tile `tile` of the array; segmented: work item `tile` is tile tk of a segment
+    struct Tile {
+        const K* in;
+        K* out;
+        uint64_t n;
+        uint32_t tk, seg, valid;
+    };
+    auto locate = [&](uint32_t tile) {
+        Tile t;
+        t.in = in_;
+        t.out = out_;
+        t.n = n_;
+        t.tk = tile;
+        t.seg = 0;
+        if constexpr (SEG) {
+            t.seg = sr.item_seg[tile];
+            t.tk = tile - sr.item_start[t.seg];
+            t.n = sr.src.len(t.seg);
+            const uint64_t a = sr.src.in_addr(t.seg), b = sr.src.aux_addr(t.seg);
+            t.in = reinterpret_cast<const K*>(sr.parity ? b : a);
+            t.out = reinterpret_cast<K*>(sr.parity ? a : b);
+            // shorter than two: sorted already, and may come without a temporary
+            if (t.n < 2) t.n = 0;
         }
-        if (tk != 0)
-            st_relaxed_u64(&status[tile * kBins + tid],
+        const uint64_t base = (uint64_t)t.tk * tile_keys;
+        const uint64_t rem = t.n > base ? t.n - base : 0;
+        t.valid = rem < (uint64_t)tile_keys ? (uint32_t)rem : tile_keys;
+        t.in += base;
+        return t;
+    };
+    K k[ITEMS];
+    // keys of warp w: tile positions [w * 32 * rows, (w + 1) * 32 * rows), row j of lane l at
+    // w * 32 * rows + 32 j + l, so rows walked in order visit keys in index order
+    auto load = [&](const Tile& t) {
+        const uint32_t rows = rows_of<BLOCK>(t.valid);
+        const uint32_t w0 = (uint32_t)warp * 32 * rows + lane;
+        if (t.valid == (uint32_t)TILE) {
+#pragma unroll
+            for (int j = 0; j < ITEMS; ++j) k[j] = __ldcs(t.in + w0 + 32 * j);
+        } else if (t.valid != 0) {  // padding re-reads the last key; it is replaced later
+#pragma unroll
+            for (int j0 = 0; j0 < ITEMS; j0 += G) {
+                if (j0 >= (int)rows) break;
+#pragma unroll
+                for (int j = j0; j < j0 + G; ++j) k[j] = __ldcs(t.in + min(w0 + 32 * j, t.valid - 1));
+            }
+        }
+    };
+
+    uint32_t tile = s_tile;
+    Tile t;
+    if (tile < tiles) {
+        t = locate(tile);
+        load(t);
+    }
+    while (tile < tiles) {
+        const int rows = (int)rows_of<BLOCK>(t.valid);
+        const uint32_t w0 = (uint32_t)warp * 32 * rows + lane;
+        // padding at the tile's end: the largest key, digit 255 after all others
+        if (t.valid == (uint32_t)rows * BLOCK) {
+#pragma unroll
+            for (int j = 0; j < ITEMS; ++j) k[j] = to_key<K, XF_IN>(k[j]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < ITEMS; ++j)
+                k[j] = w0 + 32 * j < t.valid ? to_key<K, XF_IN>(k[j]) : ~K(0);
+        }
+
+        // 1. stable ranks of the warp's rows by the current digit: wh[d] is the warp's count
+        // of digit d so far; a key's rank is that count plus its lower peers in its row. Even
+        // rows find their peers with ballots (ALU), odd rows through a table of lane masks
+        // (shared-memory atomic OR, read back, cleared by the group's highest lane): the two
+        // pipes share the work. Digit pass of 2^26 keys, all else equal: masks on every fourth
+        // row 239 us, every third 231, every second 226 (tiles of 48 rows); every second 223,
+        // two of three 227 (56 rows).
+        uint32_t rank2[ITEMS / 2];  // 16-bit ranks, two per register
+#pragma unroll
+        for (int j0 = 0; j0 < ITEMS; j0 += G) {
+            if (j0 >= rows) break;
+#pragma unroll
+            for (int j = j0; j < j0 + G; ++j) {
+                const uint32_t d = digit_of(k[j], shift);
+                uint32_t peers;
+                if (j & 1) {
+                    atomicOr(&wm[d], self);
+                    __syncwarp();
+                    peers = wm[d];
+                } else {
+                    peers = ballot_peers(d);
+                }
+                const uint32_t c = wh[d] + __popc(peers & lt);
+                __syncwarp();
+                if (peers >> lane == 1u) {  // the highest peer
+                    wh[d] = c + 1;
+                    if (j & 1) wm[d] = 0u;
+                }
+                __syncwarp();
+                rank2[j / 2] = (j & 1) ? rank2[j / 2] | (c << 16) : c;
+            }
+        }
+        __syncthreads();
+
+        // 2. per digit: counts of the warps -> exclusive over warps (in key order); tile
+        // count; publish AGG. Then the digit's start in the tile is added to every warp's
+        // offset, so the placement finds a key's slot with one table read.
+        uint32_t cnt = 0;
+        uint32_t wex[WARPS];
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) {
+            wex[w] = cnt;
+            cnt += s_wh[w * kBins + tid];
+        }
+        if (t.tk != 0)
+            st_relaxed_u64(&status[(uint64_t)tile * kBins + tid],
                            ((uint64_t)epoch << kEpochShift) | kStAgg | cnt);
-    }
-    const uint32_t loc = digit_exclusive_scan<uint32_t, BLOCK>(tid < kBins ? cnt : 0u, s_part32);
-    uint64_t start = 0;  // first tile: the digit's first output position
-    if (tk == 0) {
-        uint64_t h = 0;
-        if (tid < kBins) {
-            if constexpr (SEG) h = sr.seg_hist[(seg * sr.npos + sr.pos) * kBins + tid];
+        uint32_t claim = 0;
+        if (tid == 0) claim = atomicAdd(&counters[0], 1u);
+        const uint32_t loc = digit_exclusive_scan<uint32_t, BLOCK>(cnt, s_part32);
+        uint64_t start = 0;  // first tile: the digit's first output position
+        if (t.tk == 0) {
+            uint64_t h;
+            if constexpr (SEG) h = sr.seg_hist[((uint64_t)t.seg * sr.npos + sr.pos) * kBins + tid];
             else h = hist[tid];
+            start = digit_exclusive_scan<uint64_t, BLOCK>(h, s_part64);
         }
-        start = digit_exclusive_scan<uint64_t, BLOCK>(h, s_part64);
-    }
-    if (tid < kBins) {
-#pragma unroll 8
-        for (int w = 0; w < TABLES; ++w) s_wh[w * kBins + tid] += loc;
-    }
-    __syncthreads();
-
-    // 4a. keys in digit order in shared memory
 #pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-        const uint32_t r = s_rank[w0 + 32 * i];
-        const uint32_t d = digit_of(k[i], shift);
-        s_keys[wh[(i / STREAM_ITEMS) * kBins + d] + r] = k[i];
-    }
+        for (int w = 0; w < WARPS; ++w) s_wh[w * kBins + tid] = wex[w] + loc;
+        if (tid == 0) s_tile = claim;
+        __syncthreads();
 
-    // 3b. look-back, one thread per digit. The words of the kLookWindow nearest unvisited
-    // predecessors are loaded together, so one round trip to L2 covers several tiles; they
-    // are then consumed in order until an inclusive count ends the walk.
-    if (tid < kBins) {
+        // 3. keys in digit order in shared memory. (The empty asm keeps the compiler from
+        // holding every key's digit in a register since the ranking.)
+#pragma unroll
+        for (int j0 = 0; j0 < ITEMS; j0 += G) {
+            if (j0 >= rows) break;
+            uint32_t slot[G];
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                const int j = j0 + g;
+                K key = k[j];
+                if constexpr (sizeof(K) == 8) asm volatile("" : "+l"(key));
+                else asm volatile("" : "+r"(key));
+                const uint32_t r = (j & 1) ? rank2[j / 2] >> 16 : rank2[j / 2] & 0xffffu;
+                slot[g] = wh[digit_of(key, shift)] + r;
+            }
+#pragma unroll
+            for (int g = 0; g < G; ++g) s_keys[slot[g]] = k[j0 + g];
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = lane; i < kBins; i += 32) wh[i] = 0u;
+
+        // the next tile's keys are on their way while this one looks back and is written
+        const uint32_t next = s_tile;
+        Tile tn = t;
+        if (next < tiles) {
+            tn = locate(next);
+            load(tn);
+        }
+
+        // 4. look-back, one thread per digit. The words of the kLookWindow nearest unvisited
+        // predecessors are loaded together, so one round trip to L2 covers several tiles; they
+        // are then consumed in order until an inclusive count ends the walk.
         uint64_t excl = start;
-        if (tk != 0) {  // (segmented: the walk ends at the segment's first tile, always INC)
+        if (t.tk != 0) {  // (segmented: the walk ends at the segment's first tile, always INC)
             bool done = false;
             for (int64_t j = (int64_t)tile - 1; !done && j >= 0; j -= kLookWindow) {
                 uint64_t w[kLookWindow];
@@ -392,40 +432,79 @@ __global__ void __launch_bounds__(RadixShape<K>::BLOCK, RadixShape<K>::CTAS)
                 }
             }
         }
-        st_relaxed_u64(&status[tile * kBins + tid],
+        st_relaxed_u64(&status[(uint64_t)tile * kBins + tid],
                        ((uint64_t)epoch << kEpochShift) | kStInc | ((excl + cnt) & kValMask));
         // output position of tile-sorted index x: goff[d] + x (excl >= loc always)
         s_goff[tid] = excl - loc;
         s_goff32[tid] = (uint32_t)(excl - loc);
-    }
-    __syncthreads();
+        __syncthreads();
 
-    // 4b. each digit's run to its global offset (32-bit offsets when they fit: one
-    // shared-memory wavefront per 32 keys instead of two)
-    const bool off32 = n <= 0xffffffffull;
+        // 5. each digit's run to its global offset
+        bool bad = false;  // an output position outside the array: skipped and reported
+        if (t.n <= 0xffffffffull && t.valid == (uint32_t)TILE) {  // whole tile, 32-bit offsets
+            const uint32_t n32 = (uint32_t)t.n;
 #pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        const uint32_t x = (uint32_t)j * BLOCK + tid;
-        if (x < valid) {
-            const K key = s_keys[x];
-            const uint32_t d = digit_of(key, shift);
-            const uint64_t pos = off32 ? (uint64_t)(s_goff32[d] + x) : s_goff[d] + x;
-            if (pos < n) out[pos] = from_key<K, XF_OUT>(key);
-            else *err = kErrRadixRange;
+            for (int j0 = 0; j0 < ITEMS; j0 += G) {
+                K key[G];
+                uint32_t pos[G];
+#pragma unroll
+                for (int g = 0; g < G; ++g) key[g] = s_keys[(uint32_t)(j0 + g) * BLOCK + tid];
+#pragma unroll
+                for (int g = 0; g < G; ++g)
+                    pos[g] = s_goff32[digit_of(key[g], shift)] + (uint32_t)(j0 + g) * BLOCK + tid;
+#pragma unroll
+                for (int g = 0; g < G; ++g) {
+                    if (pos[g] < n32) t.out[pos[g]] = from_key<K, XF_OUT>(key[g]);
+                    else bad = true;
+                }
+            }
+        } else {
+#pragma unroll 4
+            for (uint32_t x = tid; x < t.valid; x += BLOCK) {
+                const K key = s_keys[x];
+                const uint64_t pos = s_goff[digit_of(key, shift)] + x;
+                if (pos < t.n) t.out[pos] = from_key<K, XF_OUT>(key);
+                else bad = true;
+            }
         }
+        if (bad) *err = kErrRadixRange;
+        tile = next;
+        t = tn;
     }
     if (tid == 0) persistent_exit(counters);
+}
+
+// CTAs of a digit pass that can be resident at once: its grid.
+template <typename K>
+uint64_t radix_resident() {
+    return (uint64_t)RadixShape<K>::CTAS * device_info().sm_count;
+}
+
+// Rows per warp of a tile (BLOCK x rows keys): the largest tile, cut so that the tiles fill
+// whole waves of the resident CTAs (2^22 uint32 keys: 106 us against 122 with full tiles, the
+// last wave nearly empty); arrays of less than a wave get smaller tiles on more SMs.
+template <typename K>
+uint32_t radix_rows(uint64_t n) {
+    constexpr uint64_t BLOCK = RadixShape<K>::BLOCK, ITEMS = RadixShape<K>::ITEMS;
+    const uint64_t res = radix_resident<K>();
+    const uint64_t waves = (n + BLOCK * ITEMS * res - 1) / (BLOCK * ITEMS * res);
+    uint64_t rows = (n + BLOCK * res * waves - 1) / (BLOCK * res * waves);
+    rows = (rows + kRowStep - 1) / kRowStep * kRowStep;
+    return (uint32_t)(rows < ITEMS ? rows : ITEMS);
 }
 
 template <typename K, int XF_IN, int XF_OUT>
 bool launch_pass(const K* in, K* out, uint64_t n, int shift, const unsigned long long* hist,
                  uint64_t* status, uint32_t epoch, uint32_t* counters, volatile int32_t* err,
-                 uint64_t tiles, cudaStream_t s) {
+                 uint64_t tiles, uint32_t rows, cudaStream_t s) {
     constexpr size_t smem = radix_smem<K>();
     if (!smem_opt_in<k_radix_pass<K, XF_IN, XF_OUT>>(smem))
         return cuda_ok(cudaGetLastError(), "k_radix_pass shared-memory opt-in");
-    k_radix_pass<K, XF_IN, XF_OUT><<<(unsigned)tiles, RadixShape<K>::BLOCK, smem, s>>>(
-        in, out, n, shift, hist, status, epoch, tiles, counters, err, SegRadix{});
+    const uint64_t res = radix_resident<K>();
+    k_radix_pass<K, XF_IN, XF_OUT>
+        <<<(unsigned)(tiles < res ? tiles : res), RadixShape<K>::BLOCK, smem, s>>>(
+            in, out, n, shift, hist, status, epoch, (uint32_t)tiles, rows, counters, err,
+            SegRadix{});
     return true;
 }
 
@@ -520,8 +599,11 @@ bool launch_seg_pass(const SegRadix& sr, int shift, uint64_t* status, uint32_t* 
     constexpr size_t smem = radix_smem<K>();
     if (!smem_opt_in<k_radix_pass<K, XF_IN, XF_OUT, true>>(smem))
         return cuda_ok(cudaGetLastError(), "k_radix_pass shared-memory opt-in");
-    k_radix_pass<K, XF_IN, XF_OUT, true><<<(unsigned)items_cap, RadixShape<K>::BLOCK, smem, s>>>(
-        nullptr, nullptr, 0, shift, nullptr, status, 0, items_cap, counters, err, sr);
+    const uint64_t res = radix_resident<K>();
+    k_radix_pass<K, XF_IN, XF_OUT, true>
+        <<<(unsigned)(items_cap < res ? items_cap : res), RadixShape<K>::BLOCK, smem, s>>>(
+            nullptr, nullptr, 0, shift, nullptr, status, 0, 0, RadixShape<K>::ITEMS, counters, err,
+            sr);
     return true;
 }
 
@@ -615,8 +697,9 @@ bool seg_radix_sort_keys(Workspace& ws, SegSrc src, uint64_t count, uint64_t S, 
 template <typename K, int XF>
 bool radix_sort_keys(Workspace& ws, void* d_data, uint64_t n, int p0 = 0) {
     constexpr int P = sizeof(K);
-    constexpr int TILE = RadixShape<K>::BLOCK * RadixShape<K>::ITEMS;
-    const uint64_t tiles = (n + TILE - 1) / TILE;
+    const uint32_t rows = radix_rows<K>(n);
+    const uint64_t tile = (uint64_t)RadixShape<K>::BLOCK * rows;
+    const uint64_t tiles = (n + tile - 1) / tile;
     if (tiles > 0x7fffffffull || n > kValMask) {
         set_error(PARALLAX_ERR_INVALID_ARGUMENT, "sort: too many elements");
         return false;
@@ -662,13 +745,13 @@ bool radix_sort_keys(Workspace& ws, void* d_data, uint64_t n, int p0 = 0) {
             ProfScope prof(ws, "k_radix_pass", 2 * n * sizeof(K));
             if (p == p0)
                 ok = launch_pass<K, XF, 0>(src, dst, n, 8 * p, hp, status, ep0 + p, counters, err,
-                                           tiles, s);
+                                           tiles, rows, s);
             else if (p == P - 1)
                 ok = launch_pass<K, 0, XF>(src, dst, n, 8 * p, hp, status, ep0 + p, counters, err,
-                                           tiles, s);
+                                           tiles, rows, s);
             else
                 ok = launch_pass<K, 0, 0>(src, dst, n, 8 * p, hp, status, ep0 + p, counters, err,
-                                          tiles, s);
+                                          tiles, rows, s);
         }
         if (!ok) return false;
         count_launch();
