@@ -31,6 +31,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include "../pdl.cuh"
 #include "../runtime.hpp"
 #include "../segplan.cuh"
 #include "../sortkey.cuh"
@@ -232,10 +233,11 @@ __global__ void __launch_bounds__(RadixShape<K>::BLOCK, RadixShape<K>::CTAS)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t lt = lanemask_lt();
     const uint32_t self = 1u << lane;
-    if (tid == 0) s_tile = atomicAdd(&counters[0], 1u);
     uint32_t* const wh = s_wh + warp * kBins;
     uint32_t* const wm = s_wh + (WARPS + warp) * kBins;
     for (int i = lane; i < kBins; i += 32) wh[i] = wm[i] = 0u;
+    dependent_prologue();
+    if (tid == 0) s_tile = atomicAdd(&counters[0], 1u);
     const uint32_t tiles = SEG ? sr.item_start[sr.S] : tiles_;
     const uint32_t epoch = SEG ? *sr.epoch_base + sr.pos : epoch_;
     const uint32_t tile_keys = BLOCK * tile_rows;
@@ -482,11 +484,14 @@ uint64_t radix_resident() {
 
 // Rows per warp of a tile (BLOCK x rows keys): the largest tile, cut so that the tiles fill
 // whole waves of the resident CTAs (2^22 uint32 keys: 106 us against 122 with full tiles, the
-// last wave nearly empty); arrays of less than a wave get smaller tiles on more SMs.
+// last wave nearly empty). An array that fits one tile per SM gets smaller tiles, one on every
+// SM: two per SM make the look-back longer than the ranking they save (2^20 uint32 keys 60 us
+// at two tiles per SM, 56 at one; 300,001 int64 keys 92 and 82).
 template <typename K>
 uint32_t radix_rows(uint64_t n) {
     constexpr uint64_t BLOCK = RadixShape<K>::BLOCK, ITEMS = RadixShape<K>::ITEMS;
-    const uint64_t res = radix_resident<K>();
+    const uint64_t sms = device_info().sm_count;
+    const uint64_t res = n <= BLOCK * ITEMS * sms ? sms : radix_resident<K>();
     const uint64_t waves = (n + BLOCK * ITEMS * res - 1) / (BLOCK * ITEMS * res);
     uint64_t rows = (n + BLOCK * res * waves - 1) / (BLOCK * res * waves);
     rows = (rows + kRowStep - 1) / kRowStep * kRowStep;
@@ -501,34 +506,40 @@ bool launch_pass(const K* in, K* out, uint64_t n, int shift, const unsigned long
     if (!smem_opt_in<k_radix_pass<K, XF_IN, XF_OUT>>(smem))
         return cuda_ok(cudaGetLastError(), "k_radix_pass shared-memory opt-in");
     const uint64_t res = radix_resident<K>();
-    k_radix_pass<K, XF_IN, XF_OUT>
-        <<<(unsigned)(tiles < res ? tiles : res), RadixShape<K>::BLOCK, smem, s>>>(
-            in, out, n, shift, hist, status, epoch, (uint32_t)tiles, rows, counters, err,
-            SegRadix{});
-    return true;
+    return launch_dependent(k_radix_pass<K, XF_IN, XF_OUT>, (unsigned)(tiles < res ? tiles : res),
+                            RadixShape<K>::BLOCK, smem, s, "k_radix_pass launch", in, out, n, shift,
+                            hist, status, epoch, (uint32_t)tiles, rows, counters, err, SegRadix{});
 }
 
 // ---- segmented radix sort -------------------------------------------------------------------
-// Digit counts of every segment for digit positions p0 .. P-1. A CTA takes kSegHistItems
+// Digit counts of every segment for digit positions p0 .. P-1. A CTA takes `per_cta`
 // consecutive work items (tiles; consecutive items are mostly of one segment), loads each
 // tile's keys into registers before counting them in shared memory (one memory round trip
 // per tile), and adds its counts to the segment's histogram with one global atomic per
 // nonzero (position, digit) when the segment changes and at its end: a long segment costs
-// one flush per kSegHistItems tiles instead of one per tile. seg_hist must be zero on entry.
+// one flush per `per_cta` tiles instead of one per tile. seg_hist must be zero on entry.
+// Bank conflicts of the random digits bound it (122 M records: 262 us, 3.7 TB/s); eight copies
+// of the counts, one per lane residue, measured 307 us.
 constexpr int kSegHistBlock = 512;
-constexpr int kSegHistItems = 8;
+
+// Work items per CTA: eight where that still leaves four CTAs for every SM; a short work list
+// gets a CTA per item (five 8-byte items on one CTA: 45 us, on five 9 us).
+inline uint32_t seg_hist_items(uint64_t items) {
+    const uint64_t per = items / (4ull * device_info().sm_count);
+    return per < 1 ? 1u : per > 8 ? 8u : (uint32_t)per;
+}
 
 template <typename K, int XF>
 __global__ void __launch_bounds__(kSegHistBlock)
-    k_seg_radix_hist(SegRadix sr, int p0, uint32_t* __restrict__ seg_hist) {
+    k_seg_radix_hist(SegRadix sr, int p0, uint32_t per_cta, uint32_t* __restrict__ seg_hist) {
     constexpr int P = sizeof(K);
     constexpr int TILE = RadixShape<K>::BLOCK * RadixShape<K>::ITEMS;
     constexpr int PER = (TILE + kSegHistBlock - 1) / kSegHistBlock;
     __shared__ uint32_t h[P][kBins];
     const uint32_t total = sr.item_start[sr.S];
-    const uint32_t i0 = blockIdx.x * kSegHistItems;
+    const uint32_t i0 = blockIdx.x * per_cta;
     if (i0 >= total) return;
-    const uint32_t i1 = total - i0 < (uint32_t)kSegHistItems ? total : i0 + kSegHistItems;
+    const uint32_t i1 = total - i0 < per_cta ? total : i0 + per_cta;
     const int tid = threadIdx.x;
     const int npos = P - p0;
     for (int i = tid; i < P * kBins; i += kSegHistBlock) (&h[0][0])[i] = 0u;
@@ -537,7 +548,7 @@ __global__ void __launch_bounds__(kSegHistBlock)
         __syncthreads();
         for (int i = tid; i < npos * kBins; i += kSegHistBlock) {
             uint32_t& c = h[p0 + i / kBins][i % kBins];
-            if (c) atomicAdd(&seg_hist[(seg * npos + i / kBins) * kBins + i % kBins], c);
+            if (c) atomicAdd(&seg_hist[seg * npos * kBins + i], c);
             c = 0u;
         }
         __syncthreads();
@@ -600,11 +611,10 @@ bool launch_seg_pass(const SegRadix& sr, int shift, uint64_t* status, uint32_t* 
     if (!smem_opt_in<k_radix_pass<K, XF_IN, XF_OUT, true>>(smem))
         return cuda_ok(cudaGetLastError(), "k_radix_pass shared-memory opt-in");
     const uint64_t res = radix_resident<K>();
-    k_radix_pass<K, XF_IN, XF_OUT, true>
-        <<<(unsigned)(items_cap < res ? items_cap : res), RadixShape<K>::BLOCK, smem, s>>>(
-            nullptr, nullptr, 0, shift, nullptr, status, 0, 0, RadixShape<K>::ITEMS, counters, err,
-            sr);
-    return true;
+    return launch_dependent(k_radix_pass<K, XF_IN, XF_OUT, true>,
+                            (unsigned)(items_cap < res ? items_cap : res), RadixShape<K>::BLOCK,
+                            smem, s, "segmented k_radix_pass launch", nullptr, nullptr, 0, shift,
+                            nullptr, status, 0, 0, RadixShape<K>::ITEMS, counters, err, sr);
 }
 
 // S segments (CSR offsets or descriptors, segplan.cuh), each sorted in place by digit
@@ -662,9 +672,10 @@ bool seg_radix_sort_keys(Workspace& ws, SegSrc src, uint64_t count, uint64_t S, 
             k_seg_map<256><<<seg_map_grid(S), 256, 0, s>>>(item_start, S, item_seg);
         if (!cuda_ok(cudaMemsetAsync(seg_hist, 0, hist_bytes, s), "segment histogram clear"))
             return false;
+        const uint32_t per = seg_hist_items(items_cap);
         k_seg_radix_hist<K, XF>
-            <<<(unsigned)((items_cap + kSegHistItems - 1) / kSegHistItems), kSegHistBlock, 0, s>>>(
-                sr, p0, seg_hist);
+            <<<(unsigned)((items_cap + per - 1) / per), kSegHistBlock, 0, s>>>(sr, p0, per,
+                                                                                 seg_hist);
         k_seg_radix_epoch<<<1, 256, 0, s>>>(counters, npos, status, words);
         for (int p = p0; p < P; ++p) {
             SegRadix q = sr;

@@ -23,6 +23,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include "../pdl.cuh"
 #include "../runtime.hpp"
 #include "../segplan.cuh"
 #include "../sortkey.cuh"
@@ -341,6 +342,7 @@ k_merge(const K* __restrict__ src, K* __restrict__ dst, uint64_t n, uint64_t L, 
     constexpr int OT = kBlock * SortShape<K>::ITEMS;
     __shared__ __align__(16) K sm[staged_elems<K>(OT)];
     __shared__ uint64_t s_split[2 * TPC];
+    dependent_prologue();
     const uint64_t tile0 = (uint64_t)blockIdx.x * tpc;
     const int ntiles = (int)(tiles - tile0 < (uint64_t)tpc ? tiles - tile0 : tpc);
     const int warp = threadIdx.x >> 5;
@@ -426,18 +428,19 @@ bool sort_keys(Workspace& ws, void* d_data, uint64_t n) {
             ProfScope prof(ws, "k_merge", 2 * n * sizeof(K));
             // four tiles per CTA from 2048 tiles (512 CTAs) up, one below
             volatile int32_t* err = &ws.d_slot->spin_error;
+            const bool last = pass == passes;
+            bool ok;
             if (tiles >= 2048) {
                 const unsigned grid = (unsigned)((tiles + kTilesPerCta - 1) / kTilesPerCta);
-                if (pass == passes)
-                    k_merge<K, XF, true, kTilesPerCta><<<grid, kBlock, 0, s>>>(cur, nxt, n, L, tiles, err);
-                else
-                    k_merge<K, XF, false, kTilesPerCta><<<grid, kBlock, 0, s>>>(cur, nxt, n, L, tiles, err);
+                ok = launch_dependent(last ? k_merge<K, XF, true, kTilesPerCta>
+                                           : k_merge<K, XF, false, kTilesPerCta>,
+                                      grid, kBlock, 0, s, "k_merge launch", cur, nxt, n, L, tiles, err);
             } else {
-                if (pass == passes)
-                    k_merge<K, XF, true, 1><<<(unsigned)tiles, kBlock, 0, s>>>(cur, nxt, n, L, tiles, err);
-                else
-                    k_merge<K, XF, false, 1><<<(unsigned)tiles, kBlock, 0, s>>>(cur, nxt, n, L, tiles, err);
+                ok = launch_dependent(last ? k_merge<K, XF, true, 1> : k_merge<K, XF, false, 1>,
+                                      (unsigned)tiles, kBlock, 0, s, "k_merge launch", cur, nxt, n, L,
+                                      tiles, err);
             }
+            if (!ok) return false;
         }
         count_launch(1);
         cur = nxt;
@@ -628,10 +631,10 @@ bool seg_sort_dispatch(Workspace& ws, DType t, const SegSrc& src, uint64_t count
 // Sizes from which the radix sort (a histogram launch plus one pass per key byte) beats the
 // merge sort (a tile-sort launch plus log2(tiles) merge passes). PARALLAX_SORT=merge or
 // =radix forces one path (read on every call). Both paths timed on B200 (random keys):
-// 4-byte 2^19 radix 0.074 / merge 0.062 ms, 2^20 0.082 / 0.088, 2^21 0.100 / 0.125;
-// 8-byte 2^19 0.134 / 0.099 ms, 2^20 0.139 / 0.143, 2^21 0.185 / 0.206.
-constexpr size_t kRadixMin4 = size_t(1) << 20;
-constexpr size_t kRadixMin8 = size_t(1) << 20;
+// us, radix / merge: 4-byte 100,003 keys 37.9 / 36.9, 300,001 45.1 / 48.1, 2^20 56.3 / 69.4;
+// 8-byte 300,001 82.9 / 56.4, 500,001 93.2 / 75.7, 700,001 102.5 / 110.6, 2^20 114.5 / 135.1.
+constexpr size_t kRadixMin4 = size_t(1) << 18;
+constexpr size_t kRadixMin8 = size_t(5) << 17;
 
 size_t sort_radix_min(DType t) { return dtype_size(t) == 4 ? kRadixMin4 : kRadixMin8; }
 
