@@ -164,7 +164,7 @@ static bool regrow(Workspace& ws, void** buf, size_t* cap_io, size_t bytes, size
 }
 
 char* Workspace::scratch(uint64_t tiles) {
-    size_t bytes = kScratchSmall + tiles * kStatusEntry;
+    size_t bytes = kScratchSmall + (tiles << status_shift(tiles)) * kStatusEntry;
     if (bytes <= scratch_cap) return static_cast<char*>(d_scratch);
     // Zeroed: look-back status words then read as "not ready" for every epoch, and the
     // self-resetting ticket counters start at zero.

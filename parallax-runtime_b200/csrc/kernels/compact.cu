@@ -386,7 +386,7 @@ k_compact_persistent(const T* in, T* out, uint64_t n, uint64_t num_tiles, PredDe
         const uint32_t cnt = rem < (uint64_t)TILE ? (uint32_t)rem : (uint32_t)TILE;
         const uint32_t bulk = bulk_elems<T>(cnt);
         if (cnt < (uint32_t)TILE || bulk < cnt) {  // the last tile: ragged end and padding
-            fill_ragged<T, TILE, kBlock>(buf, in, base, cnt, bulk);
+            fill_ragged<T, kBlock>(buf, in, base, cnt, bulk);
             __syncthreads();
         }
         compact_tile<T, MODE, true>(buf, bars[b], parity, sm, cur, base, cnt, prev, out, n,
@@ -462,7 +462,7 @@ bool compact_typed(Workspace& ws, CompactMode mode, const Pred& pr, const void* 
             : launch_count_if(ws, dtype_of<T>(), pr, d_in, n, reinterpret_cast<uint64_t*>(nt));
         if (!ok) return false;
     }
-    auto ts = tile_status_at<uint64_t>(scratch, ws.next_epoch(), &ws.d_slot->spin_error);
+    auto ts = tile_status_at<uint64_t>(scratch, ws.next_epoch(), &ws.d_slot->spin_error, tiles);
     // bulk copies only from HBM; the page-locked host mirror (small coherent operands,
     // whole-heap capture) takes plain loads
     const bool bulk = reinterpret_cast<uintptr_t>(d_in) % 16 == 0 && !arena_contains(d_in);

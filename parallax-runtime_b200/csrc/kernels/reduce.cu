@@ -188,6 +188,11 @@ k_reduce(const T* __restrict__ in, uint64_t n, uint64_t head, Xf xf, Op op, A id
     for (int u = 1; u < kUnroll; ++u) a = op(a, acc[u]);
 
     a = block_fold(a, op, ident);
+    if (gridDim.x == 1) {  // nothing to fold: no partial, fence and ticket (1000
+                           // fp32, synchronous call: 13.2 -> 11.8 us)
+        if (threadIdx.x == 0) store_result(out, (R)a);
+        return;
+    }
     __shared__ bool s_last;
     if (threadIdx.x == 0) {
         partials[blockIdx.x] = a;

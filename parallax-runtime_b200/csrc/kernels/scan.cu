@@ -6,18 +6,14 @@
 // shaders/scan_add.comp:14-19); exclusive adds a shift pass writing
 // out[i] = init + incl[i-1] (kernel_launcher.cpp:1346-1475).
 //
-// Here: one launch, one 512-thread CTA per 112 KiB tile (two per SM), in blockIdx order.
-// Each CTA
-//   1. stages its tile as two 56 KiB sub-tiles (512 threads x 7 x 16 bytes), one bulk
-//      copy (cp.async.bulk) and one mbarrier each, so 112 KiB per CTA are in flight at once
-//      and work starts when the first sub-tile lands (tiles.cuh),
-//   2. sums 28 (4-byte) or 14 (8-byte) consecutive elements per thread per sub-tile
-//      (rows of 112 bytes, an odd number of 16-byte words: conflict-free 128-bit shared
-//      loads),
-//   3. scans row totals with warp shuffles and the 32 (sub-tile, warp) totals in one warp,
-//   4. gets the tile's exclusive prefix by decoupled look-back (lookback.cuh),
-//   5. rescans each row, writes results into the staged tile and stores it with one bulk
-//      copy.
+// Here: one launch. 16-byte-aligned device operands go through a persistent pipeline, one
+// warp-specialised CTA per SM (k_scan_pipe): tiles are bulk-loaded (cp.async.bulk) into a ring of
+// buffers, summed and published as they land, looked back (lookback.cuh) while later tiles load,
+// scanned in place and bulk-stored. Operands that are not aligned or lie in the host mirror, scans
+// whose copies overlap their tiles, and the allocation-free entry point take one 512-thread CTA
+// per 112 KiB tile (two per SM), in blockIdx order (k_scan): stage, sum, look back, rescan, store.
+// Rows are 28 (4-byte) or 14 (8-byte) consecutive elements per thread (112 bytes, an odd number
+// of 16-byte words: conflict-free 128-bit shared loads).
 // HBM traffic is the algorithmic minimum: n*s read + n*s written.
 // Accumulation: fp32 data is scanned per thread in fp32 (28 terms per sub-tile) and carried
 // across threads, warps and tiles in fp64; integers wrap around in their unsigned type.
@@ -80,7 +76,7 @@ struct ScanShape {
 // row from shared memory, scans it and writes the results in place. The caller has
 // staged the tile (bulk part arriving on bars[] with `parity`, ragged part filled) and
 // stores it afterwards.
-template <typename T, bool EXCL, bool BULK>
+template <typename T, bool EXCL, bool BULK, int NSUB>
 __device__ __forceinline__ void scan_tile(T* buf, uint64_t* bars, uint32_t parity,
                                           typename ScanTypes<T>::A* s_tot, uint64_t tile,
                                           typename ScanTypes<T>::A init,
@@ -93,13 +89,13 @@ __device__ __forceinline__ void scan_tile(T* buf, uint64_t* bars, uint32_t parit
     constexpr int ITEMS = ScanShape<T>::ITEMS;
     constexpr int SUB = ScanShape<T>::SUB;
     constexpr int WARPS = kBlock / 32;
-    static_assert(kSub * WARPS == 32, "one lane per (sub-tile, warp)");
+    static_assert(NSUB * WARPS <= 32, "one lane per (sub-tile, warp)");
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
     // ---- phase 1: row totals of every sub-tile ----
-    A tex[kSub];  // exclusive prefix of this thread's row within its warp, per sub-tile
+    A tex[NSUB];  // exclusive prefix of this thread's row within its warp, per sub-tile
 #pragma unroll
-    for (int s = 0; s < kSub; ++s) {
+    for (int s = 0; s < NSUB; ++s) {
         if constexpr (BULK) wait_bar(&bars[s], parity, ts.err);
         const uint4* row = reinterpret_cast<const uint4*>(buf + s * SUB + tid * ITEMS);
         L sum = L(0);
@@ -118,22 +114,22 @@ __device__ __forceinline__ void scan_tile(T* buf, uint64_t* bars, uint32_t parit
     __syncthreads();
     // Every warp scans the 32 (sub-tile, warp) totals itself (identical shuffle sequence,
     // identical result), then the whole CTA runs the look-back.
-    A woff[kSub];  // offset of this warp's rows within the tile, per sub-tile
+    A woff[NSUB];  // offset of this warp's rows within the tile, per sub-tile
     A agg;
     {
-        const A v = s_tot[lane];
+        const A v = lane < NSUB * WARPS ? s_tot[lane] : A(0);
         const A vi = warp_inclusive_scan(v, OpSum());
         agg = shfl_idx(vi, 31);
         A vex = shfl_up(vi, 1);
         if (lane == 0) vex = A(0);
 #pragma unroll
-        for (int s = 0; s < kSub; ++s) woff[s] = shfl_idx(vex, s * WARPS + warp);
+        for (int s = 0; s < NSUB; ++s) woff[s] = shfl_idx(vex, s * WARPS + warp);
     }
     const A prefix = lookback_cta<A, kBlock, true>(ts, tile, agg, red, first);
 
     // ---- phase 2: scan each row and write the results in place ----
 #pragma unroll
-    for (int s = 0; s < kSub; ++s) {
+    for (int s = 0; s < NSUB; ++s) {
         A tb = (prefix + woff[s]) + tex[s];
         if constexpr (EXCL) tb = init + tb;
         uint4* row = reinterpret_cast<uint4*>(buf + s * SUB + tid * ITEMS);
@@ -162,7 +158,7 @@ __device__ __forceinline__ void scan_tile(T* buf, uint64_t* bars, uint32_t parit
         if constexpr (BULK) {
             // with sub_out: each sub-tile's bulk store leaves as soon as the sub-tile is
             // written, so its shared-memory read overlaps the next sub-tile's rescan
-            if (sub_out && s + 1 < kSub) {
+            if (sub_out && s + 1 < NSUB) {
                 fence_proxy_async_smem();
                 __syncthreads();
                 const uint32_t lo = (uint32_t)s * SUB, hi = bulk < lo + SUB ? bulk : lo + SUB;
@@ -177,7 +173,7 @@ __device__ __forceinline__ void scan_tile(T* buf, uint64_t* bars, uint32_t parit
     __syncthreads();
     if constexpr (BULK) {
         if (sub_out) {
-            const uint32_t lo = (uint32_t)(kSub - 1) * SUB;
+            const uint32_t lo = (uint32_t)(NSUB - 1) * SUB;
             if (tid == 0 && bulk > lo) {
                 bulk_store(sub_out + lo, buf + lo, (bulk - lo) * (uint32_t)sizeof(T));
                 bulk_commit();
@@ -186,24 +182,25 @@ __device__ __forceinline__ void scan_tile(T* buf, uint64_t* bars, uint32_t parit
     }
 }
 
-// One CTA per 112 KiB tile, in blockIdx order: unaligned operands (BULK = false) and the
-// allocation-free entry point.
+// One CTA per tile of NSUB 56 KiB sub-tiles, in blockIdx order: arrays of less than a wave,
+// unaligned operands (BULK = false), scans that overlap their copies and the allocation-free entry
+// point.
 // `tile0` is the first tile of this launch: a scan launched in chunks (so its copies can
 // overlap its tiles) passes each chunk's first tile, and every chunk shares one look-back
 // epoch, so the first tile of a chunk looks back into the chunks before it.
 // With `claim`, a CTA takes its tile from an atomic counter instead of its blockIdx (see
 // tile_claim()).
-template <typename T, bool EXCL, bool BULK>
+template <typename T, bool EXCL, bool BULK, int NSUB>
 __global__ void __launch_bounds__(kBlock, kCtasPerSm)
 k_scan(const T* in, T* out, uint64_t n,  // in == out allowed (in-place ABI scan)
        typename ScanTypes<T>::A init, TileStatus<typename ScanTypes<T>::A> ts, uint64_t tile0,
        uint32_t* claim) {
     using A = typename ScanTypes<T>::A;
     constexpr int SUB = ScanShape<T>::SUB;
-    constexpr int TILE = ScanShape<T>::TILE;
+    constexpr int TILE = NSUB * SUB;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     T* buf = reinterpret_cast<T*>(smem_raw);
-    __shared__ __align__(8) uint64_t bars[kSub];
+    __shared__ __align__(8) uint64_t bars[NSUB];
     __shared__ A s_tot[32];
     __shared__ A s_red[kBlock / 32 + 1];
     __shared__ int s_first[kBlock / 32];
@@ -213,9 +210,9 @@ k_scan(const T* in, T* out, uint64_t n,  // in == out allowed (in-place ABI scan
     const uint64_t base = tile * (uint64_t)TILE;
     const uint64_t rem = n - base;
     const uint32_t cnt = rem < (uint64_t)TILE ? (uint32_t)rem : (uint32_t)TILE;
-    const uint32_t bulk = stage_tile<T, SUB, kSub, kBlock, BULK>(buf, bars, in, base, cnt);
+    const uint32_t bulk = stage_tile<T, SUB, NSUB, kBlock, BULK>(buf, bars, in, base, cnt);
     __syncthreads();
-    scan_tile<T, EXCL, BULK>(buf, bars, 0, s_tot, tile, init, ts, s_red, s_first,
+    scan_tile<T, EXCL, BULK, NSUB>(buf, bars, 0, s_tot, tile, init, ts, s_red, s_first,
                              BULK ? out + base : nullptr, bulk);
     for (uint32_t e = bulk + tid; e < cnt; e += kBlock) out[base + e] = buf[e];
     if constexpr (BULK) {
@@ -224,106 +221,243 @@ k_scan(const T* in, T* out, uint64_t n,  // in == out allowed (in-place ABI scan
     if (claim && tid == 0) persistent_exit(claim);
 }
 
-// Persistent CTAs (two per SM) with two tile buffers each: the bulk copies of the next
-// claimed tile fill one buffer while the current tile is scanned out of the other, so
-// every SM keeps ~96 KiB of loads in flight. Operands 16-byte aligned.
-template <typename T, bool EXCL>
-__global__ void __launch_bounds__(kBlock, 2)
-k_scan_persistent(const T* in, T* out, uint64_t n, uint64_t num_tiles,
-                  typename ScanTypes<T>::A init, TileStatus<typename ScanTypes<T>::A> ts,
-                  uint32_t* counters) {
-    using A = typename ScanTypes<T>::A;
-    constexpr int SUB = ScanShape<T>::SUB;
-    constexpr int TILE = ScanShape<T>::TILE;
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    T* const buf0 = reinterpret_cast<T*>(smem_raw);  // buffer b at buf0 + b * TILE
-    __shared__ __align__(8) uint64_t bars[2][kSub];
-    __shared__ A s_tot[32];
-    __shared__ A s_red[kBlock / 32 + 1];
-    __shared__ int s_first[kBlock / 32];
-    __shared__ uint32_t s_tile[2];
-    const int tid = threadIdx.x;
+// Persistent pipeline without CTA-wide barriers. Operands 16-byte aligned.
+//   mover      claims a tile, bulk-loads it into a free buffer, bulk-stores it when every
+//              scanning warp has written it, and reuses the buffer
+//   sum warps  totals of the scanning warps' parts of a tile as soon as it lands; its aggregate
+//              is published at once, whatever the CTA's earlier tiles still wait for
+//   look-back  the tile's prefix: walk over earlier tiles, offset of every scanning warp
+//   scan warps results, written in place
+// What bounds it is HBM: at 2^28 fp32 / int32 elements 338 / 328 us (6.35 / 6.56 TB/s, 0.97 /
+// 1.00 of a plain copy) against 422 / 407 for one CTA per 112 KiB tile, whose load, look-back and
+// store follow one another. Its look-back is a chain through L2, so what matters is that a tile's
+// aggregate never waits for anything but its own load (sums in the scan warps, behind the tile
+// before: 3,500 us, each CTA in turn waiting for the others' queues) and that few polls meet at
+// one L2 line (TileStatus). Measured on the fp32 scan, us: four 56 KiB buffers on one CTA 338,
+// three 461, four 28 KiB buffers on two CTAs 348; sum warps 8 / 4 338 / 348; look-back warps 1 / 2
+// 338 / 350; entries per lane and round of the walk 1 / 2 / 4 338 / 371 / 372.
+constexpr int kPipeWarps = 16;   // scan warps
+constexpr int kPipeStages = 4;   // tile buffers
+constexpr int kSumWarps = 8;
+constexpr int kPipeBlock = (kPipeWarps + kSumWarps + 2) * 32;
 
+template <typename T>
+struct PipeShape {
+    static constexpr int V = 16 / sizeof(T);
+    static constexpr int ITEMS = kVpt * V;
+    static constexpr int TILE = kPipeWarps * 32 * ITEMS;
+    static constexpr size_t SMEM = (size_t)kPipeStages * TILE * sizeof(T);
+};
+
+template <typename T, bool EXCL>
+__global__ void __launch_bounds__(kPipeBlock, 1)
+k_scan_pipe(const T* in, T* out, uint64_t n, uint32_t num_tiles,
+            typename ScanTypes<T>::A init, TileStatus<typename ScanTypes<T>::A> ts,
+            uint32_t* counters) {
+    using L = typename ScanTypes<T>::L;
+    using A = typename ScanTypes<T>::A;
+    constexpr int V = PipeShape<T>::V, ITEMS = PipeShape<T>::ITEMS, TILE = PipeShape<T>::TILE;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    T* const bufs = reinterpret_cast<T*>(smem_raw);
+    __shared__ __align__(8) uint64_t full[kPipeStages], summed[kPipeStages], ready[kPipeStages],
+        written[kPipeStages];
+    __shared__ A s_tot[kPipeStages][kPipeWarps], s_off[kPipeStages][kPipeWarps], s_agg[kPipeStages];
+    __shared__ uint32_t s_tile[kPipeStages];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
-#pragma unroll
-        for (int b = 0; b < 2; ++b)
-#pragma unroll
-            for (int s = 0; s < kSub; ++s) mbar_init(&bars[b][s], 1);
-        fence_mbar_init();
-        const uint32_t t0 = atomicAdd(&counters[0], 1u);
-        s_tile[0] = t0;
-        if (t0 < num_tiles) {
-            const uint64_t base = (uint64_t)t0 * TILE;
-            const uint64_t rem = n - base;
-            issue_tile<T, SUB, kSub>(buf0, bars[0], in, base,
-                                     rem < (uint64_t)TILE ? (uint32_t)rem : (uint32_t)TILE);
+        for (int s = 0; s < kPipeStages; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&summed[s], 1);
+            mbar_init(&ready[s], 1);
+            mbar_init(&written[s], kPipeWarps);
         }
+        fence_mbar_init();
     }
     __syncthreads();
-    for (uint32_t it = 0;; ++it) {
-        const int b = it & 1;
-        const uint32_t parity = (it >> 1) & 1u;
-        const uint32_t cur = s_tile[b];
-        if (cur >= num_tiles) break;
-        if (tid == 0) {  // prefetch: claim the next tile and start its copies
-            bulk_wait_read_all();  // the previous tile's store has left the other buffer
+    auto count_of = [&](uint32_t t) {
+        const uint64_t rem = n - (uint64_t)t * TILE;
+        return rem < (uint64_t)TILE ? (uint32_t)rem : (uint32_t)TILE;
+    };
+
+    if (warp < kPipeWarps) {
+        const uint32_t row0 = (uint32_t)tid * ITEMS;
+        for (uint32_t it = 0;; ++it) {
+            const uint32_t b = it % kPipeStages, ph = (it / kPipeStages) & 1u;
+            wait_bar(&full[b], ph, ts.err);
+            if (s_tile[b] >= num_tiles) break;
+            uint4* row = reinterpret_cast<uint4*>(bufs + b * TILE + row0);
+            L x[ITEMS];
+#pragma unroll
+            for (int v = 0; v < kVpt; ++v) {
+                const uint4 r = row[v];
+                const T* e = reinterpret_cast<const T*>(&r);
+#pragma unroll
+                for (int k = 0; k < V; ++k) x[v * V + k] = (L)e[k];
+            }
+#pragma unroll
+            for (int j = 1; j < ITEMS; ++j) x[j] = x[j - 1] + x[j];
+            A tex = shfl_up(warp_inclusive_scan((A)x[ITEMS - 1], OpSum()), 1);
+            if (lane == 0) tex = A(0);
+            wait_bar(&ready[b], ph, ts.err);
+            A tb = s_off[b][warp] + tex;
+            if constexpr (EXCL) tb = init + tb;
+#pragma unroll
+            for (int v = 0; v < kVpt; ++v) {
+                uint4 r;
+                T* e = reinterpret_cast<T*>(&r);
+#pragma unroll
+                for (int k = 0; k < V; ++k) {
+                    const int j = v * V + k;
+                    if constexpr (EXCL) e[k] = (T)(j == 0 ? tb : tb + (A)x[j - 1]);
+                    else e[k] = (T)(tb + (A)x[j]);
+                }
+                row[v] = r;
+            }
             fence_proxy_async_smem();
-            const uint32_t nxt = atomicAdd(&counters[0], 1u);
-            s_tile[b ^ 1] = nxt;
-            if (nxt < num_tiles) {
-                const uint64_t nbase = (uint64_t)nxt * TILE;
-                const uint64_t nrem = n - nbase;
-                issue_tile<T, SUB, kSub>(buf0 + (size_t)(b ^ 1) * TILE, bars[b ^ 1], in, nbase,
-                                         nrem < (uint64_t)TILE ? (uint32_t)nrem : (uint32_t)TILE);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&written[b]);
+        }
+    } else if (warp < kPipeWarps + kSumWarps) {
+        const int sw = warp - kPipeWarps;
+        for (uint32_t it = 0;; ++it) {
+            const uint32_t b = it % kPipeStages, ph = (it / kPipeStages) & 1u;
+            wait_bar(&full[b], ph, ts.err);
+            const uint32_t t = s_tile[b];
+            if (t >= num_tiles) break;
+            const uint32_t cnt = count_of(t);
+#pragma unroll
+            for (int part = sw; part < kPipeWarps; part += kSumWarps) {
+                const uint32_t row0 = (uint32_t)(part * 32 + lane) * ITEMS;
+                const uint4* row = reinterpret_cast<const uint4*>(bufs + b * TILE + row0);
+                L sum = L(0);
+                if (cnt == (uint32_t)TILE) {
+#pragma unroll
+                    for (int v = 0; v < kVpt; ++v) {
+                        const uint4 r = row[v];
+                        const T* e = reinterpret_cast<const T*>(&r);
+#pragma unroll
+                        for (int k = 0; k < V; ++k) sum = sum + (L)e[k];
+                    }
+                } else {  // the last tile: what lies beyond the array counts as zero
+                    for (int j = 0; j < ITEMS; ++j)
+                        if (row0 + j < cnt) sum = sum + (L)bufs[b * TILE + row0 + j];
+                }
+                const A tot = warp_reduce((A)sum, OpSum());
+                if (lane == 0) s_tot[b][part] = tot;
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(kSumWarps * 32) : "memory");
+            if (sw == 0) {
+                const A v = lane < kPipeWarps ? s_tot[b][lane] : A(0);
+                const A vi = warp_inclusive_scan(v, OpSum());
+                const A agg = shfl_idx(vi, 31);
+                A vex = shfl_up(vi, 1);
+                if (lane == 0) {
+                    vex = A(0);
+                    publish_aggregate(ts, t, agg);
+                    s_agg[b] = agg;
+                }
+                if (lane < kPipeWarps) s_off[b][lane] = vex;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&summed[b]);
             }
         }
-        T* buf = buf0 + (size_t)b * TILE;
-        const uint64_t base = (uint64_t)cur * TILE;
-        const uint64_t rem = n - base;
-        const uint32_t cnt = rem < (uint64_t)TILE ? (uint32_t)rem : (uint32_t)TILE;
-        const uint32_t bulk = bulk_elems<T>(cnt);
-        if (cnt < (uint32_t)TILE || bulk < cnt) {  // the last tile: ragged end and padding
-            fill_ragged<T, TILE, kBlock>(buf, in, base, cnt, bulk);
-            __syncthreads();
+    } else if (warp == kPipeWarps + kSumWarps) {
+        for (uint32_t it = 0;; ++it) {
+            const uint32_t b = it % kPipeStages, ph = (it / kPipeStages) & 1u;
+            wait_bar(&full[b], ph, ts.err);
+            const uint32_t t = s_tile[b];
+            if (t >= num_tiles) break;
+            wait_bar(&summed[b], ph, ts.err);
+            const A prefix = lookback_warp<A>(ts, t, s_agg[b]);
+            if (lane < kPipeWarps) s_off[b][lane] = prefix + s_off[b][lane];
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ready[b]);
         }
-        scan_tile<T, EXCL, true>(buf, bars[b], parity, s_tot, cur, init, ts, s_red, s_first);
-        if (tid == 0 && bulk) {
-            bulk_store(out + base, buf, bulk * (uint32_t)sizeof(T));
-            bulk_commit();
+    } else if (lane == 0) {
+        auto load = [&](uint32_t b, uint32_t t) {
+            s_tile[b] = t;
+            if (t >= num_tiles) {
+                mbar_arrive(&full[b]);
+                return;
+            }
+            const uint64_t base = (uint64_t)t * TILE;
+            const uint32_t cnt = count_of(t), bulk = bulk_elems<T>(cnt);
+            T* const buf = bufs + b * TILE;
+            for (uint32_t e = bulk; e < cnt; ++e) buf[e] = in[base + e];
+            mbar_arrive_expect_tx(&full[b], bulk * (uint32_t)sizeof(T));
+            if (bulk) bulk_load(buf, in + base, bulk * (uint32_t)sizeof(T), &full[b]);
+        };
+        // One claim at a time, so the CTAs' first tiles interleave: tiles claimed in a row would
+        // be loaded in a row, and every other CTA's first look-back would wait for the last.
+        for (uint32_t b = 0; b < kPipeStages; ++b) {
+            if (b) wait_bar(&full[b - 1], 0, ts.err);
+            load(b, atomicAdd(&counters[0], 1u));
         }
-        for (uint32_t e = bulk + tid; e < cnt; e += kBlock) out[base + e] = buf[e];
-        __syncthreads();  // s_tile / s_tot / plain reads of buf done before the next round
-    }
-    if (tid == 0) {
-        bulk_wait_read_all();
+        for (uint32_t it = 0;; ++it) {
+            const uint32_t b = it % kPipeStages;
+            const uint32_t t = s_tile[b];
+            if (t >= num_tiles) break;
+            const uint32_t next = atomicAdd(&counters[0], 1u);
+            wait_bar(&written[b], (it / kPipeStages) & 1u, ts.err);
+            const uint64_t base = (uint64_t)t * TILE;
+            const uint32_t cnt = count_of(t), bulk = bulk_elems<T>(cnt);
+            const T* const buf = bufs + b * TILE;
+            if (bulk) {
+                bulk_store(out + base, buf, bulk * (uint32_t)sizeof(T));
+                bulk_commit();
+            }
+            for (uint32_t e = bulk; e < cnt; ++e) out[base + e] = buf[e];
+            bulk_wait_read_all();
+            load(b, next);
+        }
         persistent_exit(counters);
     }
 }
 
 // Launches tiles [tile0, tile0 + count).
-template <typename T, bool EXCL, bool BULK>
+template <typename T, bool EXCL, bool BULK, int NSUB = kSub>
 bool launch_tiles_single(const T* in, T* out, uint64_t n, typename ScanTypes<T>::A init,
                          TileStatus<typename ScanTypes<T>::A> ts, uint64_t count,
                          cudaStream_t s, uint64_t tile0 = 0, uint32_t* claim = nullptr) {
-    if (!smem_opt_in<k_scan<T, EXCL, BULK>>(ScanShape<T>::SMEM))
+    constexpr size_t smem = (size_t)NSUB * ScanShape<T>::SUB * sizeof(T);
+    if (!smem_opt_in<k_scan<T, EXCL, BULK, NSUB>>(smem))
         return cuda_ok(cudaGetLastError(), "k_scan shared-memory opt-in");
-    k_scan<T, EXCL, BULK><<<(unsigned)count, kBlock, ScanShape<T>::SMEM, s>>>(
+    k_scan<T, EXCL, BULK, NSUB><<<(unsigned)count, kBlock, smem, s>>>(
         in, out, n, init, ts, tile0, PXB_TILE_CLAIM ? claim : nullptr);
     return true;
 }
 
 template <typename T, bool EXCL>
-bool launch_tiles_persistent(const T* in, T* out, uint64_t n, typename ScanTypes<T>::A init,
-                             TileStatus<typename ScanTypes<T>::A> ts, uint64_t tiles,
-                             uint32_t* counters, cudaStream_t s) {
-    constexpr size_t smem = 2 * ScanShape<T>::SMEM;
-    if (!smem_opt_in<k_scan_persistent<T, EXCL>>(smem))
-        return cuda_ok(cudaGetLastError(), "k_scan_persistent shared-memory opt-in");
-    uint64_t grid = 2ull * device_info().sm_count;
-    if (grid > tiles) grid = tiles;
-    k_scan_persistent<T, EXCL><<<(unsigned)grid, kBlock, smem, s>>>(in, out, n, tiles, init, ts,
-                                                                     counters);
+bool launch_pipe(const T* in, T* out, uint64_t n, typename ScanTypes<T>::A init,
+                 TileStatus<typename ScanTypes<T>::A> ts, uint32_t* counters, cudaStream_t s) {
+    constexpr size_t smem = PipeShape<T>::SMEM;
+    if (!smem_opt_in<k_scan_pipe<T, EXCL>>(smem))
+        return cuda_ok(cudaGetLastError(), "k_scan_pipe shared-memory opt-in");
+    const uint64_t tiles = (n + PipeShape<T>::TILE - 1) / PipeShape<T>::TILE;
+    const uint64_t res = device_info().sm_count;
+    k_scan_pipe<T, EXCL><<<(unsigned)(tiles < res ? tiles : res), kPipeBlock, smem, s>>>(
+        in, out, n, (uint32_t)tiles, init, ts, counters);
     return true;
+}
+
+// Picks the kernel of an aligned device scan by its size (in 112 KiB tiles). Up to half a tile per
+// SM: single 56 KiB sub-tiles, so twice the SMs share the work (synchronous call, 2^20 int32 / int64
+// 16.4 -> 15.0 / 18.1 -> 15.8 us, 1000 fp32 15.1 -> 13.3). Up to one wave (two tiles per SM): all
+// tiles are in flight at once anyway and the pipeline's start costs more than it saves (2^20 int32
+// 17.4 us, 100,003 fp32 18.0 against 14.6). Beyond it the pipeline (16,000,001 fp32 41.9 -> 38.4).
+template <typename T, bool EXCL>
+bool launch_scan_tiles(const T* in, T* out, uint64_t n, typename ScanTypes<T>::A init,
+                       TileStatus<typename ScanTypes<T>::A> ts, uint64_t tiles, bool bulk,
+                       uint32_t* counters, cudaStream_t s) {
+    if (!bulk) return launch_tiles_single<T, EXCL, false>(in, out, n, init, ts, tiles, s, 0, counters);
+    const uint64_t sms = device_info().sm_count;
+    if (tiles <= sms / 2) {
+        const uint64_t subs = (n + ScanShape<T>::SUB - 1) / ScanShape<T>::SUB;
+        return launch_tiles_single<T, EXCL, true, 1>(in, out, n, init, ts, subs, s, 0, counters);
+    }
+    if (tiles <= 2 * sms)
+        return launch_tiles_single<T, EXCL, true>(in, out, n, init, ts, tiles, s, 0, counters);
+    return launch_pipe<T, EXCL>(in, out, n, init, ts, counters, s);
 }
 
 template <typename T>
@@ -332,14 +466,17 @@ bool scan_typed(Workspace& ws, bool exclusive, const void* d_in, void* d_out, ui
     using A = typename ScanTypes<T>::A;
     constexpr int TILE = ScanShape<T>::TILE;
     const uint64_t tiles = (n + TILE - 1) / TILE;
-    if (tiles > 0x7fffffffull) {
+    if (n / PipeShape<T>::TILE >= 0x7fffffffull) {
         set_error(PARALLAX_ERR_INVALID_ARGUMENT, "scan: %llu elements exceed the grid limit",
                   (unsigned long long)n);
         return false;
     }
-    char* scratch = ws.scratch(tiles);
+    // both kernels' tiles: the smaller ones decide the size of the status array
+    const uint64_t status_tiles = (n + PipeShape<T>::TILE - 1) / PipeShape<T>::TILE;
+    static_assert(PipeShape<T>::TILE <= TILE, "status entries for either kernel");
+    char* scratch = ws.scratch(status_tiles);
     if (!scratch) return false;
-    auto ts = tile_status_at<A>(scratch, ws.next_epoch(), &ws.d_slot->spin_error);
+    auto ts = tile_status_at<A>(scratch, ws.next_epoch(), &ws.d_slot->spin_error, status_tiles);
     A init = A(0);
     if (exclusive && init_host) {
         T v;
@@ -356,17 +493,9 @@ bool scan_typed(Workspace& ws, bool exclusive, const void* d_in, void* d_out, ui
     cudaStream_t s = ws.stream();
     ProfScope prof(ws, exclusive ? "k_scan_exclusive" : "k_scan_inclusive", 2 * n * sizeof(T));
     uint32_t* counters = reinterpret_cast<uint32_t*>(scratch + ScratchOff::counters);
-    static const bool persistent = getenv("PARALLAX_PERSISTENT_TILES") != nullptr;
-    bool ok;
-    if (exclusive) {
-        ok = !bulk ? launch_tiles_single<T, true, false>(in, out, n, init, ts, tiles, s, 0, counters)
-           : persistent ? launch_tiles_persistent<T, true>(in, out, n, init, ts, tiles, counters, s)
-                        : launch_tiles_single<T, true, true>(in, out, n, init, ts, tiles, s, 0, counters);
-    } else {
-        ok = !bulk ? launch_tiles_single<T, false, false>(in, out, n, init, ts, tiles, s, 0, counters)
-           : persistent ? launch_tiles_persistent<T, false>(in, out, n, init, ts, tiles, counters, s)
-                        : launch_tiles_single<T, false, true>(in, out, n, init, ts, tiles, s, 0, counters);
-    }
+    const bool ok = exclusive
+        ? launch_scan_tiles<T, true>(in, out, n, init, ts, tiles, bulk, counters, s)
+        : launch_scan_tiles<T, false>(in, out, n, init, ts, tiles, bulk, counters, s);
     if (!ok) return false;
     count_launch();
     return cuda_ok(cudaGetLastError(), "k_scan launch");
@@ -399,7 +528,7 @@ bool scan_copies_typed(Workspace& ws, bool exclusive, const void* h_in, const vo
     }
     char* scratch = ws.scratch(tiles);
     if (!scratch) return false;
-    auto ts = tile_status_at<A>(scratch, ws.next_epoch(), &ws.d_slot->spin_error);
+    auto ts = tile_status_at<A>(scratch, ws.next_epoch(), &ws.d_slot->spin_error, tiles);
     A init = A(0);
     if (exclusive && init_host) {
         T v;
@@ -510,7 +639,7 @@ int check_bounded_wait(uint32_t polls) {
     cudaStream_t s = ws->stream();
     if (!cuda_ok(cudaMemsetAsync(buf, 0, 2 * TILE * sizeof(T), s), "check_bounded_wait: input"))
         return PARALLAX_ERR_CUDA;
-    auto ts = tile_status_at<A>(scratch, ws->next_epoch(), &ws->d_slot->spin_error);
+    auto ts = tile_status_at<A>(scratch, ws->next_epoch(), &ws->d_slot->spin_error, 2);
     ts.limit = polls;
     if (!launch_tiles_single<T, false, true>(buf, buf + 2 * TILE, 2 * TILE, A(0), ts, 1, s, 1))
         return last_error() ? last_error() : PARALLAX_ERR_CUDA;
@@ -573,6 +702,8 @@ bool noalloc_launch(const void* d_in, void* d_out, uint64_t n, const void* init_
     ts.e = reinterpret_cast<StatusEntry*>(scratch + 256);
     ts.epoch = epoch;
     ts.err = reinterpret_cast<int32_t*>(scratch);
+    // a line per entry as long as the fixed array holds them
+    ts.shift = tiles << kStatusLineShift <= kNoAllocTiles ? kStatusLineShift : 0u;
     A init = A(0);
     if (init_host) {
         T v;

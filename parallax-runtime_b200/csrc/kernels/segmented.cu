@@ -97,6 +97,7 @@ struct SegBuffers {
     uint64_t* partials;    // one per work item
     StatusEntry* status;   // one per work item (a buffer of its own)
     uint64_t status_cap;   // entries in that buffer
+    uint32_t status_shift; // log2 of the entries' distance
     uint32_t* counters;    // [0] claim, [1] exit, [2] epoch, [3] error
 };
 
@@ -392,10 +393,12 @@ k_segmented(SegArgs<T> a, SegBuffers b, volatile int32_t* err) {
     ts.e = b.status;
     ts.epoch = b.counters[2];
     ts.err = err;
+    ts.shift = b.status_shift;
     TileStatus<uint64_t> tsk;
     tsk.e = b.status;
     tsk.epoch = b.counters[2];
     tsk.err = err;
+    tsk.shift = b.status_shift;
 
     // Thread 0 claims the next item and loads its descriptor while the current tile is still
     // in progress, so the claim's round trip and the dependent descriptor load overlap work.
@@ -716,7 +719,8 @@ bool seg_buffers(Workspace& ws, uint64_t S, uint64_t items, SegBuffers* out) {
     const size_t need = 256 + up256((S + 1) * 4) + up256(items * 8) +
                         up256(items * sizeof(ItemDesc));
     char* p = static_cast<char*>(ws.seg(need));
-    out->status = static_cast<StatusEntry*>(ws.seg_status(items));
+    out->status_shift = status_shift(items);
+    out->status = static_cast<StatusEntry*>(ws.seg_status(items << out->status_shift));
     if (!p || !out->status) return false;
     out->status_cap = ws.seg_status_cap;
     out->counters = reinterpret_cast<uint32_t*>(p);

@@ -4,15 +4,7 @@
 // (cp.async.bulk into the CTA's own shared memory) per sub-tile, each completing on its own
 // mbarrier, so work starts when the first sub-tile lands and the whole tile's bytes are in
 // flight at once. The bulk-copied part of a tile is its 16-byte-aligned prefix; the ragged
-// end of the last tile and the padding up to the tile size are filled with plain loads
-// (padding = T(0)) by the whole CTA.
-//
-// The persistent kernels keep two tile buffers per CTA: while tile i is processed out of
-// one buffer, the bulk copies of the CTA's next tile are already filling the other.
-// Tiles are claimed from an atomic counter right before their copies are issued, and a
-// CTA processes its claims in order; the lowest unfinished tile is therefore always the
-// one its owner is processing, and it only waits on lower, finished tiles, so look-back
-// waits end whatever CTAs happen to be resident.
+// end of the last tile is filled with plain loads by the whole CTA.
 #pragma once
 
 #include <mutex>
@@ -45,12 +37,12 @@ __device__ __forceinline__ void issue_tile(T* buf, uint64_t* bars, const T* in, 
     }
 }
 
-// Whole CTA: plain loads for the part of the tile the bulk copies do not cover.
-template <typename T, int TILE, int BLOCK>
+// Whole CTA: plain loads for the part of the tile the bulk copies do not cover. What lies beyond the
+// array stays as it is: the kernels mask it, or it only follows what they keep.
+template <typename T, int BLOCK>
 __device__ __forceinline__ void fill_ragged(T* buf, const T* in, uint64_t base, uint32_t cnt,
                                             uint32_t from) {
-    for (uint32_t e = from + threadIdx.x; e < (uint32_t)TILE; e += BLOCK)
-        buf[e] = e < cnt ? in[base + e] : T(0);
+    for (uint32_t e = from + threadIdx.x; e < cnt; e += BLOCK) buf[e] = in[base + e];
 }
 
 // Non-persistent staging of one tile (used by the allocation-free path and unaligned
@@ -69,7 +61,7 @@ __device__ __forceinline__ uint32_t stage_tile(T* buf, uint64_t* bars, const T* 
             issue_tile<T, SUB, NSUB>(buf, bars, in, base, cnt);
         }
     }
-    fill_ragged<T, SUB * NSUB, BLOCK>(buf, in, base, cnt, bulk);
+    fill_ragged<T, BLOCK>(buf, in, base, cnt, bulk);
     return bulk;
 }
 
