@@ -54,6 +54,7 @@
 #include <type_traits>
 
 #include "../lookback.cuh"
+#include "../pred.cuh"
 #include "../runtime.hpp"
 #include "../segplan.cuh"
 #include "../tiles.cuh"
@@ -65,8 +66,11 @@ namespace {
 struct TileShape {
     int block, vpt;
 };
-constexpr TileShape kShapes[] = {{256, 3}, {256, 7}, {512, 7}};
-constexpr int kNumShapes = 3;
+// The last one, named by its working threads, is the pipeline of the scans and of select (k_seg_scan_pipe,
+// k_seg_select_pipe): one CTA per SM, for long segments.
+constexpr TileShape kShapes[] = {{256, 3}, {256, 7}, {512, 7}, {1024, 7}};
+constexpr int kNumShapes = 4;
+constexpr int kPipeShape = 3;
 
 enum SegOp : int { SEG_REDUCE = 0, SEG_SCAN = 1, SEG_SELECT = 2, SEG_PARTITION = 3 };
 // reduce flavours
@@ -706,6 +710,381 @@ k_segmented(SegArgs<T> a, SegBuffers b, volatile int32_t* err) {
     if (tid == 0) persistent_exit(b.counters);
 }
 
+// ---- pipelines for long segments -------------------------------------------------------------------
+// The plain scan's and compaction's persistent pipelines (scan.cu, compact.cu: roles, and why a
+// tile's aggregate is published as it lands) over work items. The mover bulk-loads the 16-byte words
+// that hold an item's elements, so element e sits at slot e + mis of the buffer, like staged tiles;
+// the few foreign elements in the first and last word are masked (a word that holds one byte of the
+// segment lies in the same page). It claims and describes an item one step before it loads it.
+// Results leave through the working warps, since an item's ends are rarely 16-byte aligned.
+// 4096 lognormal segments, 122 M elements, the kernels above (256 x 7, their best) against these, whole
+// call: fp32 exclusive scan 384 -> 203 us (4.8 TB/s), int32 298 -> 188, fp64 566 -> 332; copy_if fp32 472
+// -> 193, int32 480 -> 191, fp64 648 -> 291. Bound by HBM and, for the many one-tile segments, by the
+// mover's claim, descriptor and load of one item after the other. The tuner times both: which wins
+// for a mean length depends on how many segments are short (each costs a buffer and a pass of all warps).
+constexpr int kPipeStages = 4;
+constexpr int kScanWarps = 16, kSumWarps = 8, kSelectWarps = 15;
+
+// An item in a pipeline's buffer.
+template <typename T>
+struct PipeItem {
+    T* out;              // of the segment
+    uint64_t begin;      // the item's first element in the segment
+    uint64_t seg_len, aux;
+    uint32_t item, first, mis, len;
+    bool last;           // of its segment
+};
+
+template <typename T>
+__device__ __forceinline__ void mover_load(T* buf, uint64_t* full, PipeItem<T>& slot, uint32_t item,
+                                           uint32_t total, const ItemDesc& d, uint32_t tile) {
+    slot.item = item;
+    if (item >= total) {
+        mbar_arrive(full);
+        return;
+    }
+    const T* const src = reinterpret_cast<const T*>(d.in) + (uint64_t)d.k * tile;
+    slot.begin = (uint64_t)d.k * tile;
+    slot.len = (uint32_t)min((uint64_t)tile, d.len - slot.begin);
+    slot.mis = (uint32_t)((reinterpret_cast<uintptr_t>(src) % 16) / sizeof(T));
+    slot.out = reinterpret_cast<T*>(d.out);
+    slot.seg_len = d.len;
+    slot.aux = d.aux;
+    slot.first = d.first_item;
+    slot.last = d.k == d.seg_items - 1;
+    const uint32_t bytes = (uint32_t)((slot.mis + slot.len) * sizeof(T) + 15) / 16 * 16;
+    mbar_arrive_expect_tx(full, bytes);
+    bulk_load(buf, src - slot.mis, bytes, full);
+}
+
+// The mover's loop: one item claimed and described ahead, a buffer refilled when it is free.
+template <typename T, int SLOTS>
+__device__ __forceinline__ void mover_loop(T* bufs, uint64_t* full, uint64_t* freed, PipeItem<T>* s_it,
+                                           const SegBuffers& b, uint32_t total, uint32_t tile,
+                                           volatile int32_t* err) {
+    uint32_t next = atomicAdd(&b.counters[0], 1u);
+    ItemDesc d;
+    if (next < total) d = load_desc(b.items, next);
+    for (uint32_t it = 0;; ++it) {
+        const uint32_t s = it % kPipeStages;
+        if (it >= kPipeStages) {
+            if (s_it[s].item >= total) break;
+            wait_bar(&freed[s], (it / kPipeStages - 1) & 1u, err);
+        } else if (it) {  // the CTAs' first items interleave (see k_scan_pipe)
+            wait_bar(&full[s - 1], 0, err);
+        }
+        mover_load<T>(bufs + (size_t)s * SLOTS, &full[s], s_it[s], next, total, d, tile);
+        if (next < total) {
+            next = atomicAdd(&b.counters[0], 1u);
+            if (next < total) d = load_desc(b.items, next);
+        }
+    }
+    persistent_exit(b.counters);
+}
+
+template <typename T, int WARPS>
+struct SegPipeShape {
+    static constexpr int V = 16 / sizeof(T);
+    static constexpr int ITEMS = 7 * V;
+    static constexpr int PART = 32 * ITEMS;
+    static constexpr int SLOTS = WARPS * PART;
+    static constexpr int TILE = SLOTS - V;
+    static constexpr size_t SMEM = (size_t)kPipeStages * SLOTS * sizeof(T);
+};
+
+template <typename T, bool INCL>
+__global__ void __launch_bounds__((kScanWarps + kSumWarps + 2) * 32, 1)
+k_seg_scan_pipe(SegArgs<T> a, SegBuffers b, volatile int32_t* err) {
+    using Sh = SegPipeShape<T, kScanWarps>;
+    using A = typename SegAcc<T>::type;
+    using L = typename SegRow<T>::type;
+    constexpr int V = Sh::V, ITEMS = Sh::ITEMS, PART = Sh::PART, SLOTS = Sh::SLOTS;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    T* const bufs = reinterpret_cast<T*>(smem_raw);
+    __shared__ __align__(8) uint64_t full[kPipeStages], summed[kPipeStages], ready[kPipeStages],
+        written[kPipeStages];
+    __shared__ A s_tot[kPipeStages][kScanWarps], s_off[kPipeStages][kScanWarps], s_agg[kPipeStages];
+    __shared__ PipeItem<T> s_it[kPipeStages];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) {
+        for (int s = 0; s < kPipeStages; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&summed[s], 1);
+            mbar_init(&ready[s], 1);
+            mbar_init(&written[s], kScanWarps);
+        }
+        fence_mbar_init();
+    }
+    const uint32_t total = b.item_start[a.S];
+    TileStatus<A> ts;
+    ts.e = b.status;
+    ts.epoch = b.counters[2];
+    ts.err = err;
+    ts.shift = b.status_shift;
+    __syncthreads();
+    auto phase = [](uint32_t it) { return (it / kPipeStages) & 1u; };
+    // A thread's row of an item: slots [row0, row0 + ITEMS), foreign ones as zero.
+    auto load = [&](const T* buf, uint32_t row0, uint32_t mis, uint32_t end, T (&x)[ITEMS]) {
+        load_row<T, ITEMS, V>(buf + row0, x);
+        if (row0 < mis || row0 + ITEMS > end) {
+#pragma unroll
+            for (int j = 0; j < ITEMS; ++j)
+                if (row0 + j < mis || row0 + j >= end) x[j] = T(0);
+        }
+    };
+
+    if (warp < kScanWarps) {
+        const uint32_t row0 = (uint32_t)tid * ITEMS, w0 = (uint32_t)warp * PART;
+        for (uint32_t it = 0;; ++it) {
+            const uint32_t s = it % kPipeStages;
+            wait_bar(&full[s], phase(it), err);
+            if (s_it[s].item >= total) break;
+            const uint32_t mis = s_it[s].mis, end = mis + s_it[s].len;
+            T* const buf = bufs + (size_t)s * SLOTS;
+            T x[ITEMS];
+            load(buf, row0, mis, end, x);
+            L p[ITEMS];
+            p[0] = (L)x[0];
+#pragma unroll
+            for (int j = 1; j < ITEMS; ++j) p[j] = p[j - 1] + (L)x[j];
+            A tex = shfl_up(warp_inclusive_scan((A)p[ITEMS - 1], OpSum()), 1);
+            if (lane == 0) tex = A(0);
+            wait_bar(&ready[s], phase(it), err);
+            const A tb = (A)a.init + (s_off[s][warp] + tex);
+            uint4* row = reinterpret_cast<uint4*>(buf + row0);
+#pragma unroll
+            for (int v = 0; v < 7; ++v) {
+                T o[V];
+#pragma unroll
+                for (int q = 0; q < V; ++q) {
+                    const int j = v * V + q;
+                    if constexpr (INCL) o[q] = (T)(tb + (A)p[j]);
+                    else o[q] = (T)(j == 0 ? tb : tb + (A)p[j > 0 ? j - 1 : 0]);
+                }
+                uint4 w;
+                memcpy(&w, o, 16);
+                row[v] = w;
+            }
+            __syncwarp();
+            // the warp's part of the item: whole 16-byte words where the output has its phase
+            T* const dst = s_it[s].out + s_it[s].begin - mis;  // of slot 0
+            if (reinterpret_cast<uintptr_t>(dst) % 16 == 0) {
+#pragma unroll
+                for (int v = 0; v < 7; ++v) {
+                    const uint32_t e = w0 + (uint32_t)(v * 32 + lane) * V;
+                    if (e >= mis && e + V <= end) {
+                        *reinterpret_cast<uint4*>(dst + e) = *reinterpret_cast<const uint4*>(buf + e);
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < V; ++q)
+                            if (e + q >= mis && e + q < end) dst[e + q] = buf[e + q];
+                    }
+                }
+            } else {
+                for (uint32_t e = w0 + lane; e < w0 + PART; e += 32)
+                    if (e >= mis && e < end) dst[e] = buf[e];
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&written[s]);
+        }
+    } else if (warp < kScanWarps + kSumWarps) {
+        const int sw = warp - kScanWarps;
+        for (uint32_t it = 0;; ++it) {
+            const uint32_t s = it % kPipeStages;
+            wait_bar(&full[s], phase(it), err);
+            const uint32_t item = s_it[s].item;
+            if (item >= total) break;
+            const uint32_t mis = s_it[s].mis, end = mis + s_it[s].len;
+#pragma unroll
+            for (int part = sw; part < kScanWarps; part += kSumWarps) {
+                T x[ITEMS];
+                load(bufs + (size_t)s * SLOTS, (uint32_t)(part * 32 + lane) * ITEMS, mis, end, x);
+                L sum = (L)x[0];
+#pragma unroll
+                for (int j = 1; j < ITEMS; ++j) sum = sum + (L)x[j];
+                const A tot = warp_reduce((A)sum, OpSum());
+                if (lane == 0) s_tot[s][part] = tot;
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(kSumWarps * 32) : "memory");
+            if (sw == 0) {
+                const A v = lane < kScanWarps ? s_tot[s][lane] : A(0);
+                const A vi = warp_inclusive_scan(v, OpSum());
+                const A agg = shfl_idx(vi, 31);
+                A vex = shfl_up(vi, 1);
+                if (lane == 0) {
+                    vex = A(0);
+                    publish_aggregate(ts, item, agg, s_it[s].first);
+                    s_agg[s] = agg;
+                }
+                if (lane < kScanWarps) s_off[s][lane] = vex;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&summed[s]);
+            }
+        }
+    } else if (warp == kScanWarps + kSumWarps) {  // look-back
+        for (uint32_t it = 0;; ++it) {
+            const uint32_t s = it % kPipeStages;
+            wait_bar(&full[s], phase(it), err);
+            const uint32_t item = s_it[s].item;
+            if (item >= total) break;
+            wait_bar(&summed[s], phase(it), err);
+            const A prefix = lookback_warp<A>(ts, item, s_agg[s], s_it[s].first);
+            if (lane < kScanWarps) s_off[s][lane] = prefix + s_off[s][lane];
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ready[s]);
+        }
+    } else if (lane == 0) {
+        mover_loop<T, SLOTS>(bufs, full, written, s_it, b, total, Sh::TILE, err);
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__((kSelectWarps + 3) * 32, 1)
+k_seg_select_pipe(SegArgs<T> a, PredDev<T> pred, SegBuffers b, volatile int32_t* err) {
+    using Sh = SegPipeShape<T, kSelectWarps>;
+    constexpr int V = Sh::V, ITEMS = Sh::ITEMS, PART = Sh::PART, SLOTS = Sh::SLOTS;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    T* const bufs = reinterpret_cast<T*>(smem_raw);
+    __shared__ __align__(8) uint64_t full[kPipeStages], counted[kPipeStages], published[kPipeStages],
+        ready[kPipeStages], packed[kPipeStages];
+    __shared__ uint32_t s_flags[kPipeStages][kSelectWarps * 32];
+    __shared__ uint32_t s_tot[kPipeStages][kSelectWarps], s_before[kPipeStages][kSelectWarps];
+    __shared__ uint64_t s_prefix[kPipeStages];
+    __shared__ uint32_t s_kept[kPipeStages];
+    __shared__ PipeItem<T> s_it[kPipeStages];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) {
+        for (int s = 0; s < kPipeStages; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&counted[s], kSelectWarps);
+            mbar_init(&published[s], 1);
+            mbar_init(&ready[s], 1);
+            mbar_init(&packed[s], kSelectWarps);
+        }
+        fence_mbar_init();
+    }
+    const uint32_t total = b.item_start[a.S];
+    TileStatus<uint64_t> ts;
+    ts.e = b.status;
+    ts.epoch = b.counters[2];
+    ts.err = err;
+    ts.shift = b.status_shift;
+    __syncthreads();
+    auto phase = [](uint32_t it) { return (it / kPipeStages) & 1u; };
+    auto landed = [&](uint64_t* bar, uint32_t parity) {  // warp-uniform (see k_compact_pipe)
+        if (!__any_sync(0xffffffffu, mbar_test_wait(bar, parity))) return false;
+        wait_bar(bar, parity, err);
+        return true;
+    };
+
+    if (warp < kSelectWarps) {
+        const uint32_t row0 = (uint32_t)tid * ITEMS, w0 = (uint32_t)warp * PART;
+        uint32_t ci = 0, pi = 0;  // items counted and packed by this warp so far
+        bool more = true;
+        uint32_t spins = 0;
+        while (more || pi < ci) {
+            if (more && ci - pi < kPipeStages && landed(&full[ci % kPipeStages], phase(ci))) {
+                spins = 0;
+                const uint32_t s = ci % kPipeStages;
+                if (s_it[s].item >= total) {
+                    more = false;
+                    continue;
+                }
+                const uint32_t mis = s_it[s].mis, end = mis + s_it[s].len;
+                T x[ITEMS];
+                load_row<T, ITEMS, V>(bufs + (size_t)s * SLOTS + row0, x);
+                uint32_t f = pred.template flags<ITEMS>(x, 0);
+                if (row0 + ITEMS > end) f &= row0 >= end ? 0u : (1u << (end - row0)) - 1u;
+                if (row0 < mis) f &= ~((1u << (mis - row0)) - 1u);
+                s_flags[s][tid] = f;
+                const uint32_t tot = warp_reduce((uint32_t)__popc(f), OpSum());
+                if (lane == 0) {
+                    s_tot[s][warp] = tot;
+                    mbar_arrive(&counted[s]);
+                }
+                ++ci;
+                continue;
+            }
+            if (pi < ci && landed(&ready[pi % kPipeStages], phase(pi))) {
+                spins = 0;
+                const uint32_t s = pi % kPipeStages;
+                T* const part = bufs + (size_t)s * SLOTS + w0;
+                const uint32_t f = s_flags[s][tid];
+                T x[ITEMS];
+                load_row<T, ITEMS, V>(bufs + (size_t)s * SLOTS + row0, x);
+                const uint32_t c = __popc(f);
+                const uint32_t incl = warp_inclusive_scan(c, OpSum());
+                const uint32_t kept = shfl_idx(incl, 31);
+                const uint64_t dst = s_prefix[s] + s_before[s][warp];
+                T* const out = s_it[s].out;
+                const uint64_t seg_len = s_it[s].seg_len;
+                __syncwarp();  // every row is in registers before the part is overwritten
+                uint32_t r = incl - c;
+#pragma unroll
+                for (int j = 0; j < ITEMS; ++j)
+                    if (f >> j & 1u) part[r++] = x[j];
+                __syncwarp();
+                if (kept != 0 && dst + kept <= seg_len) {  // in steps of whole 128-byte lines
+                    constexpr int LINE = 128 / sizeof(T);
+                    T* const o = out + dst;
+                    const int skew = (int)((reinterpret_cast<uintptr_t>(o) / sizeof(T)) % LINE);
+                    int i = lane - skew;
+                    if (i >= 0 && i < (int)kept) o[i] = part[i];
+#pragma unroll 4
+                    for (i += 32; i < (int)kept; i += 32) if (i >= 0) o[i] = part[i];
+                } else if (kept != 0) {
+                    *err = 3;  // only after a failed wait: never out of range
+                }
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&packed[s]);
+                ++pi;
+                continue;
+            }
+            if (++spins > kSpinLimit) {
+                *err = 2;
+                break;
+            }
+            nanosleep_ns(32);
+        }
+    } else if (warp == kSelectWarps) {  // publisher
+        for (uint32_t it = 0;; ++it) {
+            const uint32_t s = it % kPipeStages;
+            wait_bar(&full[s], phase(it), err);
+            const uint32_t item = s_it[s].item;
+            if (item >= total) break;
+            wait_bar(&counted[s], phase(it), err);
+            const uint32_t v = lane < kSelectWarps ? s_tot[s][lane] : 0u;
+            const uint32_t vi = warp_inclusive_scan(v, OpSum());
+            if (lane < kSelectWarps) s_before[s][lane] = vi - v;
+            if (lane == 31) {
+                publish_aggregate<uint64_t>(ts, item, vi, s_it[s].first);
+                s_kept[s] = vi;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&published[s]);
+        }
+    } else if (warp == kSelectWarps + 1) {  // look-back
+        for (uint32_t it = 0;; ++it) {
+            const uint32_t s = it % kPipeStages;
+            wait_bar(&full[s], phase(it), err);
+            const uint32_t item = s_it[s].item;
+            if (item >= total) break;
+            wait_bar(&published[s], phase(it), err);
+            const uint64_t kept = s_kept[s];
+            const uint64_t prefix = lookback_warp<uint64_t>(ts, item, kept, s_it[s].first);
+            if (lane == 0) {
+                s_prefix[s] = prefix;
+                if (s_it[s].last) *reinterpret_cast<uint64_t*>(s_it[s].aux) = prefix + kept;
+                mbar_arrive(&ready[s]);
+            }
+        }
+    } else if (lane == 0) {
+        mover_loop<T, SLOTS>(bufs, full, packed, s_it, b, total, Sh::TILE, err);
+    }
+}
+
 // ---- host side: buffers, tuner, graphs ------------------------------------------------------------
 size_t up256(size_t v) { return (v + 255) / 256 * 256; }
 
@@ -794,13 +1173,8 @@ bool launch_fold(Workspace& ws, const SegBuffers& b, uint64_t S, int red) {
     return cuda_ok(cudaGetLastError(), "segmented fold launch");
 }
 
-template <typename T, int BLOCK, int VPT>
-bool enqueue_shape(Workspace& ws, const SegCall& c, const SegBuffers& b) {
-    using Sh = SegShape<T, BLOCK, VPT>;
-    constexpr int TILE = Sh::TILE;
-    cudaStream_t s = ws.stream();
-    volatile int32_t* err = &ws.d_slot->spin_error;
-    const uint64_t items_cap = items_bound(c, TILE);
+template <typename T>
+SegArgs<T> seg_args(const SegCall& c) {
     SegArgs<T> args;
     args.src = c.src;
     args.S = c.S;
@@ -809,21 +1183,32 @@ bool enqueue_shape(Workspace& ws, const SegCall& c, const SegBuffers& b) {
     args.unique = c.unique;
     args.red = c.red;
     args.pred = make_seg_pred<T>(c.pred);
-    auto plan = [&](SegEmpty empty) {
-        if (items_cap <= kPlanItemsMax) {
-            k_seg_plan_items<256><<<1, 256, 0, s>>>(c.src, c.S, c.count, (uint32_t)TILE,
-                                                    b.item_start, b.counters, empty,
-                                                    nullptr, b.status,
-                                                    b.status_cap, err, b.items);
-            return;
-        }
-        k_seg_plan<256><<<1, 256, 0, s>>>(c.src, c.S, c.count, (uint32_t)TILE, b.item_start,
-                                          b.counters, empty, nullptr,
-                                          b.status, b.status_cap, err, nullptr);
-        const uint64_t dg = (items_cap + 255) / 256;
-        k_item_descs<<<(unsigned)(dg < 1184 ? dg : 1184), 256, 0, s>>>(c.src, c.S, b.item_start,
-                                                                        b.items);
-    };
+    return args;
+}
+
+// The work list of tiles of `tile` elements and its item descriptors.
+void seg_plan(Workspace& ws, const SegCall& c, const SegBuffers& b, uint64_t items_cap, uint32_t tile,
+              SegEmpty empty) {
+    cudaStream_t s = ws.stream();
+    volatile int32_t* err = &ws.d_slot->spin_error;
+    if (items_cap <= kPlanItemsMax) {
+        k_seg_plan_items<256><<<1, 256, 0, s>>>(c.src, c.S, c.count, tile, b.item_start, b.counters,
+                                                empty, nullptr, b.status, b.status_cap, err, b.items);
+        return;
+    }
+    k_seg_plan<256><<<1, 256, 0, s>>>(c.src, c.S, c.count, tile, b.item_start, b.counters, empty,
+                                      nullptr, b.status, b.status_cap, err, nullptr);
+    const uint64_t dg = (items_cap + 255) / 256;
+    k_item_descs<<<(unsigned)(dg < 1184 ? dg : 1184), 256, 0, s>>>(c.src, c.S, b.item_start, b.items);
+}
+
+template <typename T, int BLOCK, int VPT>
+bool enqueue_shape(Workspace& ws, const SegCall& c, const SegBuffers& b) {
+    using Sh = SegShape<T, BLOCK, VPT>;
+    constexpr int TILE = Sh::TILE;
+    const uint64_t items_cap = items_bound(c, TILE);
+    const SegArgs<T> args = seg_args<T>(c);
+    auto plan = [&](SegEmpty empty) { seg_plan(ws, c, b, items_cap, (uint32_t)TILE, empty); };
     switch (c.op) {
         case SEG_REDUCE:
             plan(c.red == RED_COUNT ? SegEmpty::ZERO_COUNT : SegEmpty::ZERO_RESULT);
@@ -849,6 +1234,49 @@ bool enqueue_shape(Workspace& ws, const SegCall& c, const SegBuffers& b) {
     }
 }
 
+// Elements of a work item of the pipeline.
+template <typename T>
+constexpr int pipe_tile(int op) {
+    return op == SEG_SCAN ? SegPipeShape<T, kScanWarps>::TILE : SegPipeShape<T, kSelectWarps>::TILE;
+}
+uint64_t shape_tile(const SegCall& c, int shape) {
+    const uint64_t es = dtype_size(c.t), V = 16 / es;
+    if (shape == kPipeShape)
+        return es == 4 ? pipe_tile<uint32_t>(c.op) : pipe_tile<uint64_t>(c.op);
+    return (uint64_t)kShapes[shape].block * kShapes[shape].vpt * V - V;
+}
+// Whether the pipeline takes the call: a scan or a select by predicate of one element-aligned array.
+bool pipe_takes(const SegCall& c) {
+    return (c.op == SEG_SCAN || (c.op == SEG_SELECT && !c.unique)) && c.src.offsets &&
+           c.src.in % dtype_size(c.t) == 0 && c.src.out % dtype_size(c.t) == 0;
+}
+
+template <typename T>
+bool enqueue_pipe(Workspace& ws, const SegCall& c, const SegBuffers& b) {
+    const uint64_t items_cap = items_bound(c, pipe_tile<T>(c.op));
+    const SegArgs<T> args = seg_args<T>(c);
+    seg_plan(ws, c, b, items_cap, (uint32_t)pipe_tile<T>(c.op),
+             c.op == SEG_SCAN ? SegEmpty::NONE : SegEmpty::ZERO_COUNT);
+    const uint64_t sms = device_info().sm_count;
+    const unsigned grid = (unsigned)(items_cap < sms ? items_cap : sms);
+    volatile int32_t* err = &ws.d_slot->spin_error;
+    if (c.op == SEG_SCAN) {
+        constexpr size_t smem = SegPipeShape<T, kScanWarps>::SMEM;
+        constexpr int threads = (kScanWarps + kSumWarps + 2) * 32;
+        if (!smem_opt_in<k_seg_scan_pipe<T, true>>(smem) || !smem_opt_in<k_seg_scan_pipe<T, false>>(smem))
+            return cuda_ok(cudaGetLastError(), "k_seg_scan_pipe shared-memory opt-in");
+        if (c.inclusive) k_seg_scan_pipe<T, true><<<grid, threads, smem, ws.stream()>>>(args, b, err);
+        else k_seg_scan_pipe<T, false><<<grid, threads, smem, ws.stream()>>>(args, b, err);
+    } else {
+        constexpr size_t smem = SegPipeShape<T, kSelectWarps>::SMEM;
+        if (!smem_opt_in<k_seg_select_pipe<T>>(smem))
+            return cuda_ok(cudaGetLastError(), "k_seg_select_pipe shared-memory opt-in");
+        k_seg_select_pipe<T><<<grid, (kSelectWarps + 3) * 32, smem, ws.stream()>>>(
+            args, make_pred<T>(c.pred), b, err);
+    }
+    return cuda_ok(cudaGetLastError(), "segmented pipeline launch");
+}
+
 template <typename T>
 bool enqueue_typed(Workspace& ws, const SegCall& c, int shape) {
     SegBuffers b;
@@ -856,6 +1284,7 @@ bool enqueue_typed(Workspace& ws, const SegCall& c, int shape) {
     switch (shape) {
         case 0: return enqueue_shape<T, 256, 3>(ws, c, b);
         case 1: return enqueue_shape<T, 256, 7>(ws, c, b);
+        case kPipeShape: return enqueue_pipe<T>(ws, c, b);
         default: return enqueue_shape<T, 512, 7>(ws, c, b);
     }
 }
@@ -928,7 +1357,7 @@ int tuned_shape(Workspace& ws, const SegCall& c) {
         std::lock_guard<std::mutex> g(g_tune_mu);
         tune_load_locked();
         auto it = g_tune->find(key);
-        if (it != g_tune->end()) return it->second;
+        if (it != g_tune->end() && (it->second != kPipeShape || pipe_takes(c))) return it->second;
     }
     if (!c.tune || (getenv("PARALLAX_TUNE") && atoi(getenv("PARALLAX_TUNE")) == 0)) {
         const uint64_t avg = c.S ? c.count / c.S : 0;  // untuned: by average segment length
@@ -941,6 +1370,7 @@ int tuned_shape(Workspace& ws, const SegCall& c) {
     float best_ms = 1e30f;
     cudaStream_t s = ws.stream();
     for (int cand = 0; cand < kNumShapes; ++cand) {
+        if (cand == kPipeShape && !pipe_takes(c)) continue;
         if (!enqueue(ws, c, cand)) break;  // warm-up (first-touch, module load)
         cudaEventRecord(e0, s);
         if (!enqueue(ws, c, cand)) break;
@@ -1009,8 +1439,7 @@ bool run(Workspace& ws, const SegCall& c, bool graph) {
     const uint64_t bytes = (c.op == SEG_SCAN || c.op == SEG_PARTITION ? 2 : 1) * c.count * es;
     ProfScope prof(ws, op_name(c), bytes);
     {  // planner (+ item descriptors unless it writes them) + the pass(es) (+ the fold)
-        const uint64_t V = 16 / es;
-        const uint64_t tile = (uint64_t)kShapes[shape].block * kShapes[shape].vpt * V - V;
+        const uint64_t tile = shape_tile(c, shape);
         const int plan = items_bound(c, tile) <= kPlanItemsMax ? 1 : 2;
         count_launch(plan + (c.op == SEG_PARTITION ? 3 : c.op == SEG_REDUCE ? 2 : 1));
     }
