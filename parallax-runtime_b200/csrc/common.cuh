@@ -120,16 +120,15 @@ struct FastMod64 {
     __host__ __device__ __forceinline__ bool eq(T x) const {
         static_assert(sizeof(T) == 8, "64-bit integers");
         const T rr = (T)r;
-        uint64_t d;
-        bool side = some;
-        if (rr == T(0)) {
-            d = x < T(0) ? 0ull - (uint64_t)x : (uint64_t)x;
-        } else if (rr > T(0)) {
-            side = side && x >= rr;
-            d = (uint64_t)x - r;
-        } else {
-            side = side && x <= rr;
-            d = r - (uint64_t)x;
+        uint64_t d = (uint64_t)x - r;  // |x - r| when x lies on r's side
+        bool side = some && (rr == T(0) || x >= rr);
+        if constexpr (T(-1) < T(0)) {
+            if (rr < T(0)) {
+                side = some && x <= rr;
+                d = 0ull - d;
+            } else if (rr == T(0) && x < T(0)) {
+                d = 0ull - d;
+            }
         }
         const uint64_t q = d * inv;
         const uint64_t rot = tz ? q >> tz | q << (64 - tz) : q;

@@ -25,6 +25,7 @@
 #include <type_traits>
 
 #include "../lookback.cuh"
+#include "../pdl.cuh"
 #include "../pred.cuh"
 #include "../runtime.hpp"
 #include "../tiles.cuh"
@@ -205,8 +206,8 @@ __device__ __forceinline__ void compact_tile(T* buf, uint64_t* bars, uint32_t pa
 template <typename T, int MODE, bool BULK, int NSUB>
 __global__ void __launch_bounds__(kBlock, kCtasPerSm)
 k_compact(const T* in, T* out, uint64_t n, PredDev<T> pred, TileStatus<uint64_t> ts,
-          const unsigned long long* __restrict__ num_true,
-          unsigned long long* __restrict__ count_out, uint32_t* claim) {
+          const unsigned long long* num_true,
+          unsigned long long* count_out, uint32_t* claim) {
     constexpr int SUB = Shape<T>::SUB;
     constexpr int TILE = NSUB * SUB;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -214,6 +215,7 @@ k_compact(const T* in, T* out, uint64_t n, PredDev<T> pred, TileStatus<uint64_t>
     __shared__ __align__(8) uint64_t bars[NSUB];
     __shared__ CompactSmem sm;
     __shared__ uint32_t s_claim;
+    dependent_prologue();
     const uint64_t tile = claim ? tile_claim(claim, s_claim) : blockIdx.x;
     const uint64_t base = tile * (uint64_t)TILE;
     const uint64_t rem = n - base;
@@ -258,8 +260,8 @@ struct PipeShape {
 template <typename T, int MODE>
 __global__ void __launch_bounds__(kPipeBlock, 1)
 k_compact_pipe(const T* in, T* out, uint64_t n, uint32_t num_tiles, PredDev<T> pred,
-               TileStatus<uint64_t> ts, const unsigned long long* __restrict__ num_true,
-               unsigned long long* __restrict__ count_out, uint32_t* counters) {
+               TileStatus<uint64_t> ts, const unsigned long long* num_true,
+               unsigned long long* count_out, uint32_t* counters) {
     using Sh = PipeShape<T>;
     constexpr int V = Sh::V, ITEMS = Sh::ITEMS, PART = Sh::PART, TILE = Sh::TILE;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -285,6 +287,7 @@ k_compact_pipe(const T* in, T* out, uint64_t n, uint32_t num_tiles, PredDev<T> p
         fence_mbar_init();
     }
     __syncthreads();
+    dependent_prologue();
     auto count_of = [&](uint32_t t) {
         const uint64_t rem = n - (uint64_t)t * TILE;
         return rem < (uint64_t)TILE ? (uint32_t)rem : (uint32_t)TILE;
@@ -473,9 +476,9 @@ bool launch_tiles(uint64_t n, cudaStream_t s, const T* in, T* out, PredDev<T> p,
     constexpr uint64_t tile = (uint64_t)NSUB * Shape<T>::SUB;
     if (!smem_opt_in<k_compact<T, MODE, BULK, NSUB>>(smem))
         return cuda_ok(cudaGetLastError(), "k_compact shared-memory opt-in");
-    k_compact<T, MODE, BULK, NSUB><<<(unsigned)((n + tile - 1) / tile), kBlock, smem, s>>>(
-        in, out, n, p, ts, nt, count_out, PXB_TILE_CLAIM ? counters : nullptr);
-    return true;
+    return launch_dependent(k_compact<T, MODE, BULK, NSUB>, (unsigned)((n + tile - 1) / tile), kBlock, smem,
+                            s, "k_compact launch", in, out, n, p, ts, nt, count_out,
+                            PXB_TILE_CLAIM ? counters : nullptr);
 }
 
 // Picks the kernel by size (in 112 KiB tiles), as the scans do: up to half a tile per SM single 56
@@ -494,9 +497,9 @@ bool launch_mode(uint64_t tiles, cudaStream_t s, bool bulk, const T* in, T* out,
     if (!smem_opt_in<k_compact_pipe<T, MODE>>(smem))
         return cuda_ok(cudaGetLastError(), "k_compact_pipe shared-memory opt-in");
     const uint64_t pipe_tiles = (n + PipeShape<T>::TILE - 1) / PipeShape<T>::TILE;
-    k_compact_pipe<T, MODE><<<(unsigned)(pipe_tiles < sms ? pipe_tiles : sms), kPipeBlock, smem, s>>>(
-        in, out, n, (uint32_t)pipe_tiles, p, ts, nt, count_out, counters);
-    return true;
+    return launch_dependent(k_compact_pipe<T, MODE>, (unsigned)(pipe_tiles < sms ? pipe_tiles : sms),
+                            kPipeBlock, smem, s, "k_compact_pipe launch", in, out, n,
+                            (uint32_t)pipe_tiles, p, ts, nt, count_out, counters);
 }
 
 template <typename T>

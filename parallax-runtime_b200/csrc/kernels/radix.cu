@@ -211,8 +211,7 @@ struct SegRadix {
 // XF_OUT restores them as they are written (the last pass writes the caller's values).
 template <typename K, int XF_IN, int XF_OUT, bool SEG = false>
 __global__ void __launch_bounds__(RadixShape<K>::BLOCK, RadixShape<K>::CTAS)
-    k_radix_pass(const K* __restrict__ in_, K* __restrict__ out_, uint64_t n_, int shift,
-                 const unsigned long long* __restrict__ hist, uint64_t* status, uint32_t epoch_,
+    k_radix_pass(const K* in_, K* out_, uint64_t n_, int shift, const unsigned long long* hist, uint64_t* status, uint32_t epoch_,
                  uint32_t tiles_, uint32_t tile_rows, uint32_t* counters, volatile int32_t* err,
                  SegRadix sr) {
     constexpr int BLOCK = RadixShape<K>::BLOCK, ITEMS = RadixShape<K>::ITEMS;

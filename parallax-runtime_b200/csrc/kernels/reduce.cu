@@ -17,6 +17,7 @@
 #include <limits>
 #include <type_traits>
 
+#include "../pdl.cuh"
 #include "../runtime.hpp"
 
 namespace pxb {
@@ -149,8 +150,9 @@ __device__ __forceinline__ void store_result(A* out, A v) { *out = v; }
 // in: n elements, the first `head` of which precede the first 16-byte boundary.
 template <typename T, typename A, typename R, typename Xf, typename Op>
 __global__ void __launch_bounds__(kBlock)
-k_reduce(const T* __restrict__ in, uint64_t n, uint64_t head, Xf xf, Op op, A ident,
-         A* __restrict__ partials, unsigned* __restrict__ ticket, R* __restrict__ out) {
+k_reduce(const T* in, uint64_t n, uint64_t head, Xf xf, Op op, A ident, A* partials, unsigned* ticket,
+         R* out) {
+    dependent_prologue();
     constexpr int V = 16 / sizeof(T);
     const uint64_t G = (uint64_t)gridDim.x * kBlock;
     const uint64_t g = (uint64_t)blockIdx.x * kBlock + threadIdx.x;
@@ -257,8 +259,10 @@ bool run(Workspace& ws, const char* name, const void* d_in, uint64_t n, Xf xf, O
     A* partials = reinterpret_cast<A*>(scratch + ScratchOff::partials);
     {
         ProfScope prof(ws, name, n * sizeof(T));
-        kernel<<<grid, kBlock, 0, ws.stream()>>>(static_cast<const T*>(d_in), n, head, xf, op,
-                                                 ident, partials, ticket, d_out);
+        if (!launch_dependent(kernel, (unsigned)grid, kBlock, 0, ws.stream(), "k_reduce launch",
+                              static_cast<const T*>(d_in), n, head, xf, op, ident, partials, ticket,
+                              d_out))
+            return false;
     }
     count_launch();
     return cuda_ok(cudaGetLastError(), "k_reduce launch");

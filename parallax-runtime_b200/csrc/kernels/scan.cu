@@ -23,6 +23,7 @@
 #include <mutex>
 
 #include "../lookback.cuh"
+#include "../pdl.cuh"
 #include "../runtime.hpp"
 #include "../tiles.cuh"
 #include "../tma.cuh"
@@ -206,6 +207,7 @@ k_scan(const T* in, T* out, uint64_t n,  // in == out allowed (in-place ABI scan
     __shared__ int s_first[kBlock / 32];
     __shared__ uint32_t s_claim;
     const int tid = threadIdx.x;
+    dependent_prologue();
     const uint64_t tile = tile0 + (claim ? tile_claim(claim, s_claim) : blockIdx.x);
     const uint64_t base = tile * (uint64_t)TILE;
     const uint64_t rem = n - base;
@@ -274,6 +276,7 @@ k_scan_pipe(const T* in, T* out, uint64_t n, uint32_t num_tiles,
         fence_mbar_init();
     }
     __syncthreads();
+    dependent_prologue();
     auto count_of = [&](uint32_t t) {
         const uint64_t rem = n - (uint64_t)t * TILE;
         return rem < (uint64_t)TILE ? (uint32_t)rem : (uint32_t)TILE;
@@ -422,9 +425,8 @@ bool launch_tiles_single(const T* in, T* out, uint64_t n, typename ScanTypes<T>:
     constexpr size_t smem = (size_t)NSUB * ScanShape<T>::SUB * sizeof(T);
     if (!smem_opt_in<k_scan<T, EXCL, BULK, NSUB>>(smem))
         return cuda_ok(cudaGetLastError(), "k_scan shared-memory opt-in");
-    k_scan<T, EXCL, BULK, NSUB><<<(unsigned)count, kBlock, smem, s>>>(
-        in, out, n, init, ts, tile0, PXB_TILE_CLAIM ? claim : nullptr);
-    return true;
+    return launch_dependent(k_scan<T, EXCL, BULK, NSUB>, (unsigned)count, kBlock, smem, s, "k_scan launch",
+                            in, out, n, init, ts, tile0, PXB_TILE_CLAIM ? claim : nullptr);
 }
 
 template <typename T, bool EXCL>
@@ -435,9 +437,8 @@ bool launch_pipe(const T* in, T* out, uint64_t n, typename ScanTypes<T>::A init,
         return cuda_ok(cudaGetLastError(), "k_scan_pipe shared-memory opt-in");
     const uint64_t tiles = (n + PipeShape<T>::TILE - 1) / PipeShape<T>::TILE;
     const uint64_t res = device_info().sm_count;
-    k_scan_pipe<T, EXCL><<<(unsigned)(tiles < res ? tiles : res), kPipeBlock, smem, s>>>(
-        in, out, n, (uint32_t)tiles, init, ts, counters);
-    return true;
+    return launch_dependent(k_scan_pipe<T, EXCL>, (unsigned)(tiles < res ? tiles : res), kPipeBlock, smem,
+                            s, "k_scan_pipe launch", in, out, n, (uint32_t)tiles, init, ts, counters);
 }
 
 // Picks the kernel of an aligned device scan by its size (in 112 KiB tiles). Up to half a tile per

@@ -54,6 +54,7 @@
 #include <type_traits>
 
 #include "../lookback.cuh"
+#include "../pdl.cuh"
 #include "../pred.cuh"
 #include "../runtime.hpp"
 #include "../segplan.cuh"
@@ -160,8 +161,8 @@ struct SegArgs {
 // Writes the descriptor of every work item (one thread per item, grid-stride): the item's
 // segment is found by binary search over the planner's item_start.
 __global__ void __launch_bounds__(256)
-k_item_descs(SegSrc src, uint64_t S, const uint32_t* __restrict__ item_start,
-             ItemDesc* __restrict__ items) {
+k_item_descs(SegSrc src, uint64_t S, const uint32_t* item_start, ItemDesc* items) {
+    dependent_prologue();
     const uint32_t total = item_start[S];
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += gridDim.x * blockDim.x) {
@@ -187,7 +188,8 @@ template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK)
 k_seg_plan_items(SegSrc src, uint64_t S, uint64_t count, uint32_t tile, uint32_t* item_start,
                  uint32_t* counters, SegEmpty empty, uint32_t* seg_zero, StatusEntry* status,
-                 uint64_t status_cap, volatile int32_t* err, ItemDesc* __restrict__ items) {
+                 uint64_t status_cap, volatile int32_t* err, ItemDesc* items) {
+    dependent_prologue();
     seg_plan_block<BLOCK>(src, S, count, tile, item_start, counters, empty, seg_zero, status,
                           status_cap, err, nullptr);
     __syncthreads();
@@ -346,6 +348,7 @@ __device__ __forceinline__ uint32_t lane_mask_lt() {
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_seg_fold(SegBuffers b, uint64_t S, int red) {
+    dependent_prologue();
     using A = typename SegAcc<T>::type;
     const uint64_t s = ((uint64_t)blockIdx.x * 256 + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -382,7 +385,7 @@ k_segmented(SegArgs<T> a, SegBuffers b, volatile int32_t* err) {
     constexpr int ITEMS = Sh::ITEMS;
     constexpr int TILE = Sh::TILE;
     constexpr int WARPS = BLOCK / 32;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    extern __shared__ __align__(128) unsigned char smem_raw[];
     T* sm = reinterpret_cast<T*>(smem_raw);
     __shared__ A red[WARPS + 1];
     __shared__ uint64_t red64[WARPS + 1];
@@ -393,6 +396,7 @@ k_segmented(SegArgs<T> a, SegBuffers b, volatile int32_t* err) {
     __shared__ uint32_t s_item;
     __shared__ T s_prev;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    dependent_prologue();
     const uint32_t total = b.item_start[a.S];
     TileStatus<A> ts;
     ts.e = b.status;
@@ -815,6 +819,7 @@ k_seg_scan_pipe(SegArgs<T> a, SegBuffers b, volatile int32_t* err) {
         }
         fence_mbar_init();
     }
+    dependent_prologue();
     const uint32_t total = b.item_start[a.S];
     TileStatus<A> ts;
     ts.e = b.status;
@@ -964,6 +969,7 @@ k_seg_select_pipe(SegArgs<T> a, PredDev<T> pred, SegBuffers b, volatile int32_t*
         }
         fence_mbar_init();
     }
+    dependent_prologue();
     const uint32_t total = b.item_start[a.S];
     TileStatus<uint64_t> ts;
     ts.e = b.status;
@@ -1162,15 +1168,15 @@ bool launch_kernel(Workspace& ws, const SegArgs<T>& args, const SegBuffers& b, u
     }
     const uint64_t resident = (uint64_t)per_sm * device_info().sm_count;
     const unsigned grid = (unsigned)(items < resident ? items : resident);
-    kfn<<<grid ? grid : 1, BLOCK, smem, ws.stream()>>>(args, b, &ws.d_slot->spin_error);
-    return cuda_ok(cudaGetLastError(), "segmented launch");
+    return launch_dependent(kfn, grid ? grid : 1, BLOCK, smem, ws.stream(), "segmented launch", args, b,
+                            &ws.d_slot->spin_error);
 }
 
 template <typename T>
 bool launch_fold(Workspace& ws, const SegBuffers& b, uint64_t S, int red) {
     const uint64_t blocks = (S * 32 + 255) / 256;
-    k_seg_fold<T><<<(unsigned)(blocks ? blocks : 1), 256, 0, ws.stream()>>>(b, S, red);
-    return cuda_ok(cudaGetLastError(), "segmented fold launch");
+    return launch_dependent(k_seg_fold<T>, (unsigned)(blocks ? blocks : 1), 256, 0, ws.stream(),
+                            "segmented fold launch", b, S, red);
 }
 
 template <typename T>
@@ -1187,19 +1193,20 @@ SegArgs<T> seg_args(const SegCall& c) {
 }
 
 // The work list of tiles of `tile` elements and its item descriptors.
-void seg_plan(Workspace& ws, const SegCall& c, const SegBuffers& b, uint64_t items_cap, uint32_t tile,
+bool seg_plan(Workspace& ws, const SegCall& c, const SegBuffers& b, uint64_t items_cap, uint32_t tile,
               SegEmpty empty) {
     cudaStream_t s = ws.stream();
     volatile int32_t* err = &ws.d_slot->spin_error;
-    if (items_cap <= kPlanItemsMax) {
-        k_seg_plan_items<256><<<1, 256, 0, s>>>(c.src, c.S, c.count, tile, b.item_start, b.counters,
-                                                empty, nullptr, b.status, b.status_cap, err, b.items);
-        return;
-    }
-    k_seg_plan<256><<<1, 256, 0, s>>>(c.src, c.S, c.count, tile, b.item_start, b.counters, empty,
-                                      nullptr, b.status, b.status_cap, err, nullptr);
+    if (items_cap <= kPlanItemsMax)
+        return launch_dependent(k_seg_plan_items<256>, 1, 256, 0, s, "segment plan launch", c.src, c.S,
+                                c.count, tile, b.item_start, b.counters, empty, nullptr, b.status,
+                                b.status_cap, err, b.items);
     const uint64_t dg = (items_cap + 255) / 256;
-    k_item_descs<<<(unsigned)(dg < 1184 ? dg : 1184), 256, 0, s>>>(c.src, c.S, b.item_start, b.items);
+    return launch_dependent(k_seg_plan<256>, 1, 256, 0, s, "segment plan launch", c.src, c.S, c.count,
+                            tile, b.item_start, b.counters, empty, nullptr, b.status, b.status_cap, err,
+                            nullptr) &&
+           launch_dependent(k_item_descs, (unsigned)(dg < 1184 ? dg : 1184), 256, 0, s,
+                            "item descriptor launch", c.src, c.S, b.item_start, b.items);
 }
 
 template <typename T, int BLOCK, int VPT>
@@ -1208,25 +1215,25 @@ bool enqueue_shape(Workspace& ws, const SegCall& c, const SegBuffers& b) {
     constexpr int TILE = Sh::TILE;
     const uint64_t items_cap = items_bound(c, TILE);
     const SegArgs<T> args = seg_args<T>(c);
-    auto plan = [&](SegEmpty empty) { seg_plan(ws, c, b, items_cap, (uint32_t)TILE, empty); };
+    auto plan = [&](SegEmpty empty) { return seg_plan(ws, c, b, items_cap, (uint32_t)TILE, empty); };
     switch (c.op) {
         case SEG_REDUCE:
-            plan(c.red == RED_COUNT ? SegEmpty::ZERO_COUNT : SegEmpty::ZERO_RESULT);
-            return launch_kernel<T, BLOCK, VPT, SEG_REDUCE>(ws, args, b, items_cap) &&
+            return plan(c.red == RED_COUNT ? SegEmpty::ZERO_COUNT : SegEmpty::ZERO_RESULT) &&
+                   launch_kernel<T, BLOCK, VPT, SEG_REDUCE>(ws, args, b, items_cap) &&
                    launch_fold<T>(ws, b, c.S, c.red);
         case SEG_SCAN:
-            plan(SegEmpty::NONE);
-            return launch_kernel<T, BLOCK, VPT, SEG_SCAN>(ws, args, b, items_cap);
+            return plan(SegEmpty::NONE) &&
+                   launch_kernel<T, BLOCK, VPT, SEG_SCAN>(ws, args, b, items_cap);
         case SEG_SELECT:
-            plan(SegEmpty::ZERO_COUNT);
-            return launch_kernel<T, BLOCK, VPT, SEG_SELECT>(ws, args, b, items_cap);
+            return plan(SegEmpty::ZERO_COUNT) &&
+                   launch_kernel<T, BLOCK, VPT, SEG_SELECT>(ws, args, b, items_cap);
         default: {
             // count pass (per-segment kept totals into the counts), then the scatter; the
             // count pass uses no look-back status, so the scatter takes the plan's epoch
             SegArgs<T> cnt = args;
             cnt.red = RED_COUNT;
-            plan(SegEmpty::ZERO_COUNT);
-            if (!launch_kernel<T, BLOCK, VPT, SEG_REDUCE>(ws, cnt, b, items_cap) ||
+            if (!plan(SegEmpty::ZERO_COUNT) ||
+                !launch_kernel<T, BLOCK, VPT, SEG_REDUCE>(ws, cnt, b, items_cap) ||
                 !launch_fold<T>(ws, b, c.S, RED_COUNT))
                 return false;
             return launch_kernel<T, BLOCK, VPT, SEG_PARTITION>(ws, args, b, items_cap);
@@ -1255,8 +1262,9 @@ template <typename T>
 bool enqueue_pipe(Workspace& ws, const SegCall& c, const SegBuffers& b) {
     const uint64_t items_cap = items_bound(c, pipe_tile<T>(c.op));
     const SegArgs<T> args = seg_args<T>(c);
-    seg_plan(ws, c, b, items_cap, (uint32_t)pipe_tile<T>(c.op),
-             c.op == SEG_SCAN ? SegEmpty::NONE : SegEmpty::ZERO_COUNT);
+    if (!seg_plan(ws, c, b, items_cap, (uint32_t)pipe_tile<T>(c.op),
+                  c.op == SEG_SCAN ? SegEmpty::NONE : SegEmpty::ZERO_COUNT))
+        return false;
     const uint64_t sms = device_info().sm_count;
     const unsigned grid = (unsigned)(items_cap < sms ? items_cap : sms);
     volatile int32_t* err = &ws.d_slot->spin_error;
@@ -1265,16 +1273,14 @@ bool enqueue_pipe(Workspace& ws, const SegCall& c, const SegBuffers& b) {
         constexpr int threads = (kScanWarps + kSumWarps + 2) * 32;
         if (!smem_opt_in<k_seg_scan_pipe<T, true>>(smem) || !smem_opt_in<k_seg_scan_pipe<T, false>>(smem))
             return cuda_ok(cudaGetLastError(), "k_seg_scan_pipe shared-memory opt-in");
-        if (c.inclusive) k_seg_scan_pipe<T, true><<<grid, threads, smem, ws.stream()>>>(args, b, err);
-        else k_seg_scan_pipe<T, false><<<grid, threads, smem, ws.stream()>>>(args, b, err);
-    } else {
-        constexpr size_t smem = SegPipeShape<T, kSelectWarps>::SMEM;
-        if (!smem_opt_in<k_seg_select_pipe<T>>(smem))
-            return cuda_ok(cudaGetLastError(), "k_seg_select_pipe shared-memory opt-in");
-        k_seg_select_pipe<T><<<grid, (kSelectWarps + 3) * 32, smem, ws.stream()>>>(
-            args, make_pred<T>(c.pred), b, err);
+        return launch_dependent(c.inclusive ? k_seg_scan_pipe<T, true> : k_seg_scan_pipe<T, false>, grid,
+                                threads, smem, ws.stream(), "segmented scan launch", args, b, err);
     }
-    return cuda_ok(cudaGetLastError(), "segmented pipeline launch");
+    constexpr size_t smem = SegPipeShape<T, kSelectWarps>::SMEM;
+    if (!smem_opt_in<k_seg_select_pipe<T>>(smem))
+        return cuda_ok(cudaGetLastError(), "k_seg_select_pipe shared-memory opt-in");
+    return launch_dependent(k_seg_select_pipe<T>, grid, (kSelectWarps + 3) * 32, smem, ws.stream(),
+                            "segmented select launch", args, make_pred<T>(c.pred), b, err);
 }
 
 template <typename T>

@@ -99,6 +99,7 @@ k_tile_sort(const K* in, K* out, uint64_t n, bool apply_inverse) {
     constexpr int TILE = kBlock * ITEMS;
     constexpr int V = 16 / sizeof(K);
     __shared__ K sm[TILE];
+    dependent_prologue();
     const int t = threadIdx.x, lane = t & 31;
     const uint64_t base = (uint64_t)blockIdx.x * TILE;
     const uint64_t rem = n - base;
@@ -336,7 +337,7 @@ static_assert(2 * kTilesPerCta <= kBlock / 32, "one warp per split");
 
 template <typename K, int XF, bool FINAL, int TPC>
 __global__ void __launch_bounds__(kBlock)
-k_merge(const K* __restrict__ src, K* __restrict__ dst, uint64_t n, uint64_t L, uint64_t tiles,
+k_merge(const K* src, K* dst, uint64_t n, uint64_t L, uint64_t tiles,
         volatile int32_t* err) {
     constexpr int tpc = TPC;
     constexpr int OT = kBlock * SortShape<K>::ITEMS;
@@ -418,7 +419,9 @@ bool sort_keys(Workspace& ws, void* d_data, uint64_t n) {
     K* cur = (passes % 2 == 0) ? data : tmp;
     {
         ProfScope prof(ws, "k_tile_sort", 2 * n * sizeof(K));
-        k_tile_sort<K, XF><<<(unsigned)tiles, kBlock, 0, s>>>(data, cur, n, passes == 0);
+        if (!launch_dependent(k_tile_sort<K, XF>, (unsigned)tiles, kBlock, 0, s, "k_tile_sort launch",
+                              data, cur, n, passes == 0))
+            return false;
     }
     count_launch();
     for (int pass = 1; pass <= passes; ++pass) {

@@ -15,6 +15,7 @@
 
 #include "common.cuh"
 #include "lookback.cuh"
+#include "pdl.cuh"
 
 namespace pxb {
 
@@ -74,7 +75,8 @@ __device__ __forceinline__ uint32_t find_segment(const uint32_t* item_start, uin
 constexpr uint64_t kInlineItems = 16384;
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK)
-k_seg_map(const uint32_t* __restrict__ item_start, uint64_t S, uint32_t* __restrict__ item_seg) {
+k_seg_map(const uint32_t* item_start, uint64_t S, uint32_t* item_seg) {
+    dependent_prologue();
     for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < S;
          s += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t a = item_start[s], b = item_start[s + 1];
@@ -183,9 +185,10 @@ __device__ __forceinline__ void seg_plan_block(SegSrc src, uint64_t S, uint64_t 
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK)
 k_seg_plan(SegSrc src, uint64_t S, uint64_t count, uint32_t tile,
-           uint32_t* __restrict__ item_start, uint32_t* __restrict__ counters, SegEmpty empty,
-           uint32_t* __restrict__ seg_zero, StatusEntry* status, uint64_t status_cap,
-           volatile int32_t* err, uint32_t* __restrict__ item_seg) {
+           uint32_t* item_start, uint32_t* counters, SegEmpty empty,
+           uint32_t* seg_zero, StatusEntry* status, uint64_t status_cap,
+           volatile int32_t* err, uint32_t* item_seg) {
+    dependent_prologue();
     seg_plan_block<BLOCK>(src, S, count, tile, item_start, counters, empty, seg_zero, status,
                           status_cap, err, item_seg);
 }
