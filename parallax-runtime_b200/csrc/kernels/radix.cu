@@ -530,7 +530,8 @@ inline uint32_t seg_hist_items(uint64_t items) {
 
 template <typename K, int XF>
 __global__ void __launch_bounds__(kSegHistBlock)
-    k_seg_radix_hist(SegRadix sr, int p0, uint32_t per_cta, uint32_t* __restrict__ seg_hist) {
+    k_seg_radix_hist(SegRadix sr, int p0, uint32_t per_cta, uint32_t tile, uint32_t* seg_hist) {
+    dependent_prologue();
     constexpr int P = sizeof(K);
     constexpr int TILE = RadixShape<K>::BLOCK * RadixShape<K>::ITEMS;
     constexpr int PER = (TILE + kSegHistBlock - 1) / kSegHistBlock;
@@ -562,9 +563,9 @@ __global__ void __launch_bounds__(kSegHistBlock)
         const uint64_t len = sr.src.len(seg);
         if (len < 2) continue;  // not sorted (see k_radix_pass)
         const uint64_t k = item - sr.item_start[seg];
-        const K* in = reinterpret_cast<const K*>(sr.src.in_addr(seg)) + k * TILE;
-        const uint64_t rem = len - k * TILE;
-        const uint32_t cnt = rem < (uint64_t)TILE ? (uint32_t)rem : (uint32_t)TILE;
+        const K* in = reinterpret_cast<const K*>(sr.src.in_addr(seg)) + k * tile;
+        const uint64_t rem = len - k * tile;
+        const uint32_t cnt = rem < (uint64_t)tile ? (uint32_t)rem : tile;
         K key[PER];
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
@@ -587,6 +588,7 @@ __global__ void __launch_bounds__(256)
     k_seg_radix_epoch(uint32_t* counters, uint32_t npass, uint64_t* status, uint64_t words) {
     __shared__ uint32_t s_base;
     __shared__ bool s_wrap;
+    dependent_prologue();
     if (threadIdx.x == 0) {
         uint32_t e = counters[2];
         if (e == 0) e = 1;  // a zeroed buffer: words of epoch 0 never match
@@ -605,7 +607,7 @@ __global__ void __launch_bounds__(256)
 
 template <typename K, int XF_IN, int XF_OUT>
 bool launch_seg_pass(const SegRadix& sr, int shift, uint64_t* status, uint32_t* counters,
-                     volatile int32_t* err, uint64_t items_cap, cudaStream_t s) {
+                     volatile int32_t* err, uint64_t items_cap, uint32_t rows, cudaStream_t s) {
     constexpr size_t smem = radix_smem<K>();
     if (!smem_opt_in<k_radix_pass<K, XF_IN, XF_OUT, true>>(smem))
         return cuda_ok(cudaGetLastError(), "k_radix_pass shared-memory opt-in");
@@ -613,7 +615,7 @@ bool launch_seg_pass(const SegRadix& sr, int shift, uint64_t* status, uint32_t* 
     return launch_dependent(k_radix_pass<K, XF_IN, XF_OUT, true>,
                             (unsigned)(items_cap < res ? items_cap : res), RadixShape<K>::BLOCK,
                             smem, s, "segmented k_radix_pass launch", nullptr, nullptr, 0, shift,
-                            nullptr, status, 0, 0, RadixShape<K>::ITEMS, counters, err, sr);
+                            nullptr, status, 0, 0, rows, counters, err, sr);
 }
 
 // S segments (CSR offsets or descriptors, segplan.cuh), each sorted in place by digit
@@ -624,8 +626,10 @@ template <typename K, int XF>
 bool seg_radix_sort_keys(Workspace& ws, SegSrc src, uint64_t count, uint64_t S, int p0,
                          bool graph) {
     constexpr int P = sizeof(K);
-    constexpr int TILE = RadixShape<K>::BLOCK * RadixShape<K>::ITEMS;
-    const uint64_t items_cap = S + count / TILE + 1;
+    // a batch of little work gets smaller tiles, as a small array does
+    const uint32_t rows = radix_rows<K>(count);
+    const uint32_t tile = RadixShape<K>::BLOCK * rows;
+    const uint64_t items_cap = S + count / tile + 1;
     const uint32_t npos = (uint32_t)(P - p0);
     if (items_cap >= 0x7fffffffull || (npos % 2) != 0) {
         set_error(PARALLAX_ERR_INVALID_ARGUMENT, "segmented sort: too many tiles");
@@ -664,31 +668,35 @@ bool seg_radix_sort_keys(Workspace& ws, SegSrc src, uint64_t count, uint64_t S, 
     ProfScope prof(ws, "segmented_radix_sort", 2 * count * sizeof(K));
     count_launch(4 + npos);
     auto enqueue = [&]() -> bool {
-        k_seg_plan<256><<<1, 256, 0, s>>>(src, S, count, (uint32_t)TILE, item_start, plan_counters,
-                                          SegEmpty::NONE, nullptr, st, ws.seg_status_cap, err,
-                                          items_cap <= kInlineItems ? item_seg : nullptr);
-        if (items_cap > kInlineItems)
-            k_seg_map<256><<<seg_map_grid(S), 256, 0, s>>>(item_start, S, item_seg);
-        if (!cuda_ok(cudaMemsetAsync(seg_hist, 0, hist_bytes, s), "segment histogram clear"))
+        if (!cuda_ok(cudaMemsetAsync(seg_hist, 0, hist_bytes, s), "segment histogram clear") ||
+            !launch_dependent(k_seg_plan<kPlanBlock>, 1, kPlanBlock, 0, s, "segment plan launch", src, S, count, tile,
+                              item_start, plan_counters, SegEmpty::NONE, nullptr, st,
+                              ws.seg_status_cap, err, items_cap <= kInlineItems ? item_seg : nullptr))
+            return false;
+        if (items_cap > kInlineItems &&
+            !launch_dependent(k_seg_map<256>, seg_map_grid(S), 256, 0, s, "segment map launch",
+                              item_start, S, item_seg))
             return false;
         const uint32_t per = seg_hist_items(items_cap);
-        k_seg_radix_hist<K, XF>
-            <<<(unsigned)((items_cap + per - 1) / per), kSegHistBlock, 0, s>>>(sr, p0, per,
-                                                                                 seg_hist);
-        k_seg_radix_epoch<<<1, 256, 0, s>>>(counters, npos, status, words);
+        if (!launch_dependent(k_seg_radix_hist<K, XF>, (unsigned)((items_cap + per - 1) / per),
+                              kSegHistBlock, 0, s, "segment histogram launch", sr, p0, per, tile,
+                              seg_hist) ||
+            !launch_dependent(k_seg_radix_epoch, 1, 256, 0, s, "segment epoch launch", counters, npos,
+                              status, words))
+            return false;
         for (int p = p0; p < P; ++p) {
             SegRadix q = sr;
             q.pos = (uint32_t)(p - p0);
             q.parity = (uint32_t)((p - p0) & 1);
             bool ok;
             if (p == p0 && p == P - 1)
-                ok = launch_seg_pass<K, XF, XF>(q, 8 * p, status, counters, err, items_cap, s);
+                ok = launch_seg_pass<K, XF, XF>(q, 8 * p, status, counters, err, items_cap, rows, s);
             else if (p == p0)
-                ok = launch_seg_pass<K, XF, 0>(q, 8 * p, status, counters, err, items_cap, s);
+                ok = launch_seg_pass<K, XF, 0>(q, 8 * p, status, counters, err, items_cap, rows, s);
             else if (p == P - 1)
-                ok = launch_seg_pass<K, 0, XF>(q, 8 * p, status, counters, err, items_cap, s);
+                ok = launch_seg_pass<K, 0, XF>(q, 8 * p, status, counters, err, items_cap, rows, s);
             else
-                ok = launch_seg_pass<K, 0, 0>(q, 8 * p, status, counters, err, items_cap, s);
+                ok = launch_seg_pass<K, 0, 0>(q, 8 * p, status, counters, err, items_cap, rows, s);
             if (!ok) return false;
         }
         return cuda_ok(cudaGetLastError(), "segmented radix sort launch");

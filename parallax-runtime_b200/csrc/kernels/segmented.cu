@@ -1198,11 +1198,11 @@ bool seg_plan(Workspace& ws, const SegCall& c, const SegBuffers& b, uint64_t ite
     cudaStream_t s = ws.stream();
     volatile int32_t* err = &ws.d_slot->spin_error;
     if (items_cap <= kPlanItemsMax)
-        return launch_dependent(k_seg_plan_items<256>, 1, 256, 0, s, "segment plan launch", c.src, c.S,
+        return launch_dependent(k_seg_plan_items<kPlanBlock>, 1, kPlanBlock, 0, s, "segment plan launch", c.src, c.S,
                                 c.count, tile, b.item_start, b.counters, empty, nullptr, b.status,
                                 b.status_cap, err, b.items);
     const uint64_t dg = (items_cap + 255) / 256;
-    return launch_dependent(k_seg_plan<256>, 1, 256, 0, s, "segment plan launch", c.src, c.S, c.count,
+    return launch_dependent(k_seg_plan<kPlanBlock>, 1, kPlanBlock, 0, s, "segment plan launch", c.src, c.S, c.count,
                             tile, b.item_start, b.counters, empty, nullptr, b.status, b.status_cap, err,
                             nullptr) &&
            launch_dependent(k_item_descs, (unsigned)(dg < 1184 ? dg : 1184), 256, 0, s,

@@ -491,8 +491,8 @@ __device__ __forceinline__ SegGeom<K> seg_geom(const SegSrc& src, const uint32_t
 
 template <typename K, int XF>
 __global__ void __launch_bounds__(kBlock)
-k_seg_tile_sort(SegSrc src, uint64_t S, const uint32_t* __restrict__ item_start,
-                const uint32_t* __restrict__ item_seg) {
+k_seg_tile_sort(SegSrc src, uint64_t S, const uint32_t* item_start, const uint32_t* item_seg) {
+    dependent_prologue();
     constexpr int ITEMS = SortShape<K>::ITEMS;
     constexpr int TILE = kBlock * ITEMS;
     __shared__ K sm[TILE];
@@ -518,8 +518,9 @@ k_seg_tile_sort(SegSrc src, uint64_t S, const uint32_t* __restrict__ item_start,
 // pass; like k_merge, warps 0 and 1 find the tile's span on the merge path first.
 template <typename K, int XF>
 __global__ void __launch_bounds__(kBlock)
-k_seg_merge(SegSrc src, uint64_t S, const uint32_t* __restrict__ item_start,
-            const uint32_t* __restrict__ item_seg, int pass, volatile int32_t* err) {
+k_seg_merge(SegSrc src, uint64_t S, const uint32_t* item_start, const uint32_t* item_seg, int pass,
+            volatile int32_t* err) {
+    dependent_prologue();
     constexpr int OT = kBlock * SortShape<K>::ITEMS;
     __shared__ __align__(16) K sm[staged_elems<K>(OT)];
     __shared__ uint64_t s_split[2];
@@ -585,18 +586,20 @@ bool seg_sort_keys(Workspace& ws, SegSrc src, uint64_t count, uint64_t S, uint64
     count_launch(3 + pass_bound);
     auto enqueue = [&] {
         cudaStream_t s = ws.stream();
-        k_seg_plan<kBlock><<<1, kBlock, 0, s>>>(src, S, count, (uint32_t)TILE, item_start, counters,
-                                                SegEmpty::NONE, nullptr, st, ws.seg_status_cap,
-                                                &ws.d_slot->spin_error,
-                                                items_cap <= kInlineItems ? item_seg : nullptr);
+        bool ok = launch_dependent(k_seg_plan<kPlanBlock>, 1, kPlanBlock, 0, s, "segment plan launch", src, S,
+                                   count, (uint32_t)TILE, item_start, counters, SegEmpty::NONE, nullptr,
+                                   st, ws.seg_status_cap, &ws.d_slot->spin_error,
+                                   items_cap <= kInlineItems ? item_seg : nullptr);
         const unsigned grid = (unsigned)items_cap;
         if (items_cap > kInlineItems)
-            k_seg_map<256><<<seg_map_grid(S), 256, 0, s>>>(item_start, S, item_seg);
-        k_seg_tile_sort<K, XF><<<grid, kBlock, 0, s>>>(src, S, item_start, item_seg);
-        for (int pass = 1; pass <= pass_bound; ++pass)
-            k_seg_merge<K, XF><<<grid, kBlock, 0, s>>>(src, S, item_start, item_seg, pass,
-                                                       &ws.d_slot->spin_error);
-        return cuda_ok(cudaGetLastError(), "segmented sort launch");
+            ok = ok && launch_dependent(k_seg_map<256>, seg_map_grid(S), 256, 0, s, "segment map launch",
+                                        item_start, S, item_seg);
+        ok = ok && launch_dependent(k_seg_tile_sort<K, XF>, grid, kBlock, 0, s, "segmented tile sort launch",
+                                    src, S, item_start, item_seg);
+        for (int pass = 1; ok && pass <= pass_bound; ++pass)
+            ok = launch_dependent(k_seg_merge<K, XF>, grid, kBlock, 0, s, "segmented merge launch", src, S,
+                                  item_start, item_seg, pass, &ws.d_slot->spin_error);
+        return ok;
     };
     if (!graph) return enqueue();
     char key[256];

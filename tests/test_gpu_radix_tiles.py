@@ -53,3 +53,26 @@ def test_segments_of_every_tile_fill(lib, px, dev):
     for s in range(len(lens)):
         a, b = int(off[s]), int(off[s + 1])
         assert np.array_equal(got[a:b], rec[a:b][np.argsort(keys[a:b], kind="stable")]), s
+
+
+@pytest.mark.parametrize("dtype", ["u32", "f64"])
+def test_small_batches_use_small_tiles(lib, px, ox, dev, monkeypatch, dtype):
+    """A batch of less than a tile per SM is cut into smaller tiles: segments around their size, sorted
+    by the radix path."""
+    monkeypatch.setenv("PARALLAX_SORT", "radix")
+    np_t = {"u32": np.uint32, "f64": np.float64}[dtype]
+    es = np.dtype(np_t).itemsize
+    rng = np.random.default_rng(12)
+    for scale in (1, 7, 30):  # 4 to 40-odd rows per warp
+        lens = [0, 1, STEP - 1, STEP, STEP + 1, 100 * STEP * scale // 7 + 5, 3, 0, 2 * STEP * scale + 1]
+        off = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint64)
+        n = int(off[-1])
+        x = rng.integers(0, 2 ** 32, n, dtype=np.uint32) if dtype == "u32" else rng.standard_normal(n)
+        d, o = dev.put(x), dev.put(off)
+        st = lib.parallax_segmented_sort(px.builtin(f"sort:{dtype}"), d.data_ptr(), n, o.data_ptr(), len(lens))
+        assert st == px.OK
+        got = dev.get(d, np_t, n)
+        for s in range(len(lens)):
+            a, b = int(off[s]), int(off[s + 1])
+            if b > a:
+                assert np.array_equal(got[a:b].view(np.uint8), ox.sort(x[a:b]).view(np.uint8)), (scale, s)
