@@ -241,9 +241,12 @@ k_compact(const T* in, T* out, uint64_t n, PredDev<T> pred, TileStatus<uint64_t>
 // What bounds it is the workers' latency chain per tile (flags 1,000 to 1,800 cycles, packing 1,200,
 // storing 900 of a 4,600-cycle period) behind HBM at 0.7 to 0.85 of the copy rate. 2^28 int32 x % 3
 // == 0 / fp32 x > 0.5 / unique, us: one CTA per 112 KiB tile 397 / 399 / 354, the same with a line per
-// look-back entry 350 / 358 / 309, this pipeline 313 / 301 / 270. 20 workers with rows of 80 bytes
-// 315 / 311 / 281, 24 with 48 bytes and five buffers 426 / 381 / 350, 20 with 112 bytes and three
-// buffers 313 / 342 / 297; counting and packing on separate warps 395 / 422 / 342.
+// look-back entry 350 / 358 / 309, this pipeline 299 / 297 / 266. Before a part was totalled with one
+// redux instead of five shuffles 313 / 301 / 270; then also 20 workers with rows of 80 bytes 315 / 311 /
+// 281, 24 with 48 bytes and five buffers 426 / 381 / 350, 20 with 112 bytes and three buffers 313 / 342
+// / 297, counting and packing on separate warps 395 / 422 / 342; now also 12 workers and five buffers
+// 326 / 315 / 295, two groups of 14 workers on alternate tiles 344 / 348 / 310, two or three look-back
+// warps or a walk that starts before the count is known 301 / 299 / 268.
 constexpr int kPipeWorkers = 15;  // 15 parts of 3.5 KiB, four tiles and their flags fit an SM
 constexpr int kPipeStages = 4;
 constexpr int kPipeBlock = (kPipeWorkers + 3) * 32;
@@ -333,7 +336,7 @@ k_compact_pipe(const T* in, T* out, uint64_t n, uint32_t num_tiles, PredDev<T> p
                 }
                 if (row0 + ITEMS > cnt) f &= row0 >= cnt ? 0u : (1u << (cnt - row0)) - 1u;
                 s_flags[b][tid] = f;
-                const uint32_t tot = warp_reduce((uint32_t)__popc(f), OpSum());
+                const uint32_t tot = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(f));
                 if (lane == 0) {
                     s_tot[b][warp] = tot;
                     mbar_arrive(&counted[b]);

@@ -1004,7 +1004,7 @@ k_seg_select_pipe(SegArgs<T> a, PredDev<T> pred, SegBuffers b, volatile int32_t*
                 if (row0 + ITEMS > end) f &= row0 >= end ? 0u : (1u << (end - row0)) - 1u;
                 if (row0 < mis) f &= ~((1u << (mis - row0)) - 1u);
                 s_flags[s][tid] = f;
-                const uint32_t tot = warp_reduce((uint32_t)__popc(f), OpSum());
+                const uint32_t tot = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(f));
                 if (lane == 0) {
                     s_tot[s][warp] = tot;
                     mbar_arrive(&counted[s]);
