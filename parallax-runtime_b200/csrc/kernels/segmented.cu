@@ -69,6 +69,7 @@ struct TileShape {
 };
 // The last one, named by its working threads, is the pipeline of the scans and of select (k_seg_scan_pipe,
 // k_seg_select_pipe): one CTA per SM, for long segments.
+// A reduce's {512, 7} is a pipeline too (k_seg_reduce_pipe).
 constexpr TileShape kShapes[] = {{256, 3}, {256, 7}, {512, 7}, {1024, 7}};
 constexpr int kNumShapes = 4;
 constexpr int kPipeShape = 3;
@@ -944,6 +945,111 @@ k_seg_scan_pipe(SegArgs<T> a, SegBuffers b, volatile int32_t* err) {
     }
 }
 
+// Reduces of long segments: the same ring, and nothing else. An item waits for no other one, so the
+// mover may claim far ahead: its first four items are dealt by CTA (a claim of four each would starve
+// the last CTAs of a short list), later ones are claimed four steps and described two steps before
+// their load, so neither round trip is on its path. Every working warp folds its part of an item
+// (vectors lane by lane: no bank conflicts), the fold warp adds the warps' results and frees the buffer.
+// It stands in for the {512, 7} shape, whose tile it has and which was never a reduce's best.
+// 4096 lognormal segments, 122 M elements, whole call, 256 x 7 (the best before) against this: fp32 121
+// -> 90 us, int32 109 -> 88 (floor 75, the planner 9), fp64 182 -> 154 (floor 149).
+constexpr int kFoldWarps = 16;
+
+template <typename T, int RED>
+__global__ void __launch_bounds__((kFoldWarps + 2) * 32, 1)
+k_seg_reduce_pipe(SegArgs<T> a, SegBuffers b, volatile int32_t* err) {
+    using Sh = SegPipeShape<T, kFoldWarps>;
+    using A = std::conditional_t<RED == RED_SUM, typename SegAcc<T>::type, T>;
+    using Op = std::conditional_t<RED == RED_SUM, OpSum, std::conditional_t<RED == RED_MAX, OpMax, OpMin>>;
+    constexpr int V = Sh::V, PART = Sh::PART, SLOTS = Sh::SLOTS;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    T* const bufs = reinterpret_cast<T*>(smem_raw);
+    __shared__ __align__(8) uint64_t full[kPipeStages], summed[kPipeStages], freed[kPipeStages];
+    __shared__ A s_tot[kPipeStages][kFoldWarps];
+    __shared__ PipeItem<T> s_it[kPipeStages];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) {
+        for (int s = 0; s < kPipeStages; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&summed[s], kFoldWarps);
+            mbar_init(&freed[s], 1);
+        }
+        fence_mbar_init();
+    }
+    dependent_prologue();
+    const uint32_t total = b.item_start[a.S];
+    __syncthreads();
+    auto phase = [](uint32_t it) { return (it / kPipeStages) & 1u; };
+    const A ident = RED == RED_SUM ? A(0) : (A)red_identity<T>(RED);
+
+    if (warp < kFoldWarps) {
+        for (uint32_t it = 0;; ++it) {
+            const uint32_t s = it % kPipeStages;
+            wait_bar(&full[s], phase(it), err);
+            if (s_it[s].item >= total) break;
+            const uint32_t mis = s_it[s].mis, end = mis + s_it[s].len, w0 = (uint32_t)warp * PART;
+            A acc = ident;
+            if (w0 < end) {  // a short item leaves the last warps nothing
+                const T* const buf = bufs + (size_t)s * SLOTS;
+#pragma unroll
+                for (int v = 0; v < 7; ++v) {
+                    const uint32_t e0 = w0 + (uint32_t)(v * 32 + lane) * V;
+                    const uint4 q = *reinterpret_cast<const uint4*>(buf + e0);
+                    T x[V];
+                    memcpy(x, &q, 16);
+#pragma unroll
+                    for (int e = 0; e < V; ++e)
+                        if (e0 + e >= mis && e0 + e < end) acc = Op()(acc, (A)x[e]);
+                }
+                acc = warp_reduce(acc, Op());
+            }
+            __syncwarp();  // every lane has read s_it[s]
+            if (lane == 0) {
+                s_tot[s][warp] = acc;
+                mbar_arrive(&summed[s]);
+            }
+        }
+    } else if (warp == kFoldWarps) {
+        for (uint32_t it = 0;; ++it) {
+            const uint32_t s = it % kPipeStages;
+            wait_bar(&full[s], phase(it), err);
+            const uint32_t item = s_it[s].item;
+            if (item >= total) break;
+            wait_bar(&summed[s], phase(it), err);
+            const A tot = warp_reduce(lane < kFoldWarps ? s_tot[s][lane] : ident, Op());
+            if (lane == 0) {
+                if (s_it[s].begin == 0 && s_it[s].last) *reinterpret_cast<T*>(s_it[s].aux) = (T)tot;
+                else put_val(&b.partials[item], tot);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&freed[s]);
+        }
+    } else if (lane == 0) {
+        static_assert(kPipeStages == 4, "the claims below are unrolled over the ring");
+        uint32_t next[4];
+        ItemDesc d[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            next[u] = blockIdx.x + u * gridDim.x;
+            if (u < 2 && next[u] < total) d[u] = load_desc(b.items, next[u]);
+        }
+        bool more = true;
+        for (uint32_t turn = 0; more; ++turn) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (!more) continue;
+                if (turn) wait_bar(&freed[u], (turn - 1) & 1u, err);
+                mover_load<T>(bufs + (size_t)u * SLOTS, &full[u], s_it[u], next[u], total, d[u], Sh::TILE);
+                more = next[u] < total;
+                if (more) next[u] = 4 * gridDim.x + atomicAdd(&b.counters[0], 1u);
+                const int w = (u + 2) % 4;
+                if (more && next[w] < total) d[w] = load_desc(b.items, next[w]);
+            }
+        }
+        persistent_exit(b.counters);
+    }
+}
+
 template <typename T>
 __global__ void __launch_bounds__((kSelectWarps + 3) * 32, 1)
 k_seg_select_pipe(SegArgs<T> a, PredDev<T> pred, SegBuffers b, volatile int32_t* err) {
@@ -1283,6 +1389,36 @@ bool enqueue_pipe(Workspace& ws, const SegCall& c, const SegBuffers& b) {
                             "segmented select launch", args, make_pred<T>(c.pred), b, err);
 }
 
+// Whether a reduce of the {512, 7} shape runs as the pipeline: sums and extremes of one
+// element-aligned array.
+bool reduce_pipe_takes(const SegCall& c) {
+    return c.op == SEG_REDUCE && c.red != RED_COUNT && c.src.offsets && c.src.in % dtype_size(c.t) == 0;
+}
+
+template <typename T, int RED>
+bool launch_reduce_pipe(Workspace& ws, const SegArgs<T>& args, const SegBuffers& b, uint64_t items) {
+    constexpr size_t smem = SegPipeShape<T, kFoldWarps>::SMEM;
+    if (!smem_opt_in<k_seg_reduce_pipe<T, RED>>(smem))
+        return cuda_ok(cudaGetLastError(), "k_seg_reduce_pipe shared-memory opt-in");
+    const uint64_t sms = device_info().sm_count;
+    const unsigned grid = (unsigned)(items < sms ? items : sms);
+    return launch_dependent(k_seg_reduce_pipe<T, RED>, grid ? grid : 1, (kFoldWarps + 2) * 32, smem, ws.stream(),
+                            "segmented reduce launch", args, b, (volatile int32_t*)&ws.d_slot->spin_error);
+}
+
+template <typename T>
+bool enqueue_reduce_pipe(Workspace& ws, const SegCall& c, const SegBuffers& b) {
+    constexpr int TILE = SegPipeShape<T, kFoldWarps>::TILE;
+    static_assert(TILE == SegShape<T, 512, 7>::TILE, "the work list is the shape's");
+    const uint64_t items_cap = items_bound(c, TILE);
+    const SegArgs<T> args = seg_args<T>(c);
+    return seg_plan(ws, c, b, items_cap, (uint32_t)TILE, SegEmpty::ZERO_RESULT) &&
+           (c.red == RED_SUM   ? launch_reduce_pipe<T, RED_SUM>(ws, args, b, items_cap)
+            : c.red == RED_MAX ? launch_reduce_pipe<T, RED_MAX>(ws, args, b, items_cap)
+                               : launch_reduce_pipe<T, RED_MIN>(ws, args, b, items_cap)) &&
+           launch_fold<T>(ws, b, c.S, c.red);
+}
+
 template <typename T>
 bool enqueue_typed(Workspace& ws, const SegCall& c, int shape) {
     SegBuffers b;
@@ -1291,7 +1427,8 @@ bool enqueue_typed(Workspace& ws, const SegCall& c, int shape) {
         case 0: return enqueue_shape<T, 256, 3>(ws, c, b);
         case 1: return enqueue_shape<T, 256, 7>(ws, c, b);
         case kPipeShape: return enqueue_pipe<T>(ws, c, b);
-        default: return enqueue_shape<T, 512, 7>(ws, c, b);
+        default:
+            return reduce_pipe_takes(c) ? enqueue_reduce_pipe<T>(ws, c, b) : enqueue_shape<T, 512, 7>(ws, c, b);
     }
 }
 
