@@ -49,8 +49,8 @@ constexpr int kEpochShift = 42;
 constexpr int kLookWindow = 4;  // predecessor words a look-back step loads at once
 
 // Keys per thread ("rows" of 32 keys per warp) of the largest tile, at two 256-thread CTAs per
-// SM. What bounds a pass is neither HBM (a fifth busy) nor one pipe, but the ALU (ballots) and
-// the shared-memory pipe (random digits) at about 70 % each, plus a cost per tile (counts,
+// SM. What bounds a pass is not HBM (a quarter busy) but the shared-memory pipe (random digits, 79 %
+// busy) and the ALU (ballots, 54 %) together, plus a cost per tile (counts,
 // digit scan, look-back) of some 4,000 cycles: large tiles of few warps win until the keys and
 // their ranks no longer fit the 128 registers. Digit pass measured on B200, 2^26 uint32 keys /
 // 2^25 int64 keys: 512 threads x 24 / 16 rows, one tile per CTA (as it was) 306 / 215 us; 256 x
