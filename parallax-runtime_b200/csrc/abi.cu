@@ -11,6 +11,7 @@
 
 #include <limits>
 
+#include "compact_shape.hpp"
 #include "parallax/kernel_abi.h"
 #include "runtime.hpp"
 

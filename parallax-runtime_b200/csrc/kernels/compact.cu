@@ -24,6 +24,7 @@
 
 #include <type_traits>
 
+#include "../compact_shape.hpp"
 #include "../lookback.cuh"
 #include "../pdl.cuh"
 #include "../pred.cuh"
@@ -34,20 +35,6 @@
 namespace pxb {
 namespace {
 
-// Tile shape (measured: 112 KiB tiles, 2 CTAs/SM); can be overridden at build time
-// (PXB_COMPACT_BLOCK / _VPT / _SUB / _CTAS) to sweep it; kSub x (kBlock / 32) must be 32.
-#ifndef PXB_COMPACT_BLOCK
-#define PXB_COMPACT_BLOCK 512
-#endif
-#ifndef PXB_COMPACT_VPT
-#define PXB_COMPACT_VPT 7
-#endif
-#ifndef PXB_COMPACT_SUB
-#define PXB_COMPACT_SUB 2
-#endif
-#ifndef PXB_COMPACT_CTAS
-#define PXB_COMPACT_CTAS 2
-#endif
 constexpr int kBlock = PXB_COMPACT_BLOCK;
 constexpr int kVpt = PXB_COMPACT_VPT;
 constexpr int kSub = PXB_COMPACT_SUB;
@@ -60,6 +47,7 @@ struct Shape {
     static constexpr int SUB = kBlock * ITEMS;
     static constexpr int TILE = kSub * SUB;
     static constexpr size_t SMEM = TILE * sizeof(T);
+    static_assert(TILE == compact_tile(sizeof(T)), "flags arrays are padded to it");
 };
 
 // Shared state of one CTA's tile processing.
@@ -247,17 +235,18 @@ k_compact(const T* in, T* out, uint64_t n, PredDev<T> pred, TileStatus<uint64_t>
 // / 297, counting and packing on separate warps 395 / 422 / 342; now also 12 workers and five buffers
 // 326 / 315 / 295, two groups of 14 workers on alternate tiles 344 / 348 / 310, two or three look-back
 // warps or a walk that starts before the count is known 301 / 299 / 268.
-constexpr int kPipeWorkers = 15;  // 15 parts of 3.5 KiB, four tiles and their flags fit an SM
+constexpr int kPipeWorkers = kCompactPipeWorkers;
 constexpr int kPipeStages = 4;
 constexpr int kPipeBlock = (kPipeWorkers + 3) * 32;
 
 template <typename T>
 struct PipeShape {
     static constexpr int V = 16 / sizeof(T);
-    static constexpr int ITEMS = 7 * V;        // odd number of 16-byte words: conflict-free rows
+    static constexpr int ITEMS = kCompactPipeVpt * V;
     static constexpr int PART = 32 * ITEMS;
     static constexpr int TILE = kPipeWorkers * PART;  // 52.5 KiB
     static constexpr size_t SMEM = (size_t)kPipeStages * TILE * sizeof(T);
+    static_assert(TILE == compact_pipe_tile(sizeof(T)), "flags arrays are padded to it");
 };
 
 template <typename T, int MODE>
@@ -563,12 +552,6 @@ bool compact_typed(Workspace& ws, CompactMode mode, const Pred& pr, const void* 
 }
 
 }  // namespace
-
-size_t compact_flags_padding(size_t n) {
-    constexpr size_t kTile = Shape<uint32_t>::TILE;  // the largest tile, in elements
-    static_assert(Shape<uint32_t>::TILE % Shape<uint64_t>::TILE == 0, "tile sizes nest");
-    return (n + kTile - 1) / kTile * kTile + 16;
-}
 
 bool launch_compact(Workspace& ws, DType t, CompactMode mode, const Pred& p, const void* d_in,
                     void* d_out, size_t n, uint64_t* d_count) {

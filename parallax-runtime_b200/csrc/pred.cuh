@@ -44,7 +44,8 @@ struct PredDev {
         switch (kind) {
             case PredKind::FLAGS:
                 // rows start at multiples of ITEMS (28 or 14), so the row's flag bytes are
-                // 4-byte (or 2-byte) aligned; the array is padded past the last tile
+                // 4-byte (or 2-byte) aligned; the array is padded to the end of the last
+                // tile of every kernel (compact_flags_padding)
                 if constexpr (ITEMS % 4 == 0) {
                     const uint32_t* w = reinterpret_cast<const uint32_t*>(fl + gi);
 #pragma unroll

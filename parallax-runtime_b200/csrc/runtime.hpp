@@ -315,9 +315,6 @@ bool launch_count_if(Workspace& ws, DType t, const Pred& p, const void* d_in, si
                      uint64_t* d_count);
 // Number of nonzero bytes of a flags array (partition with a registered `:flags` image).
 bool launch_count_flags(Workspace& ws, const uint8_t* d_flags, size_t n, uint64_t* d_count);
-// Elements a flags array written for launch_compact with PredKind::FLAGS must be padded to
-// (the compaction reads whole rows of flags; bytes past n are ignored).
-size_t compact_flags_padding(size_t n);
 // by_key: 8-byte (key << 32 | value) records sorted stably by key (sort_kv handles).
 bool launch_sort(Workspace& ws, DType t, void* d_data, size_t n, bool by_key = false);
 // Smallest array launch_sort gives to the radix sort (by default; PARALLAX_SORT overrides).
