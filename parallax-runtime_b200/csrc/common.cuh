@@ -166,7 +166,18 @@ template <> struct SumAcc<int64_t> { using type = uint64_t; };
 template <> struct SumAcc<uint64_t> { using type = uint64_t; };
 
 // ---- 16-byte streaming global loads ---------------------------------------------------
-// Read-only, no L1 allocation: every input byte of these kernels is touched once.
+// No L1 allocation: every input byte of these kernels is touched once. ldg_stream16 is a read-only
+// load, for kernels that start when everything before them has finished; ld_stream16 a coherent one,
+// for dependent launches (pdl.cuh), during whose lifetime the kernels before them still write.
+// Equally fast: 2^28 fp32 sum 158 us with either.
+__device__ __forceinline__ uint4 ld_stream16(const void* p) {
+    uint4 r;
+    asm volatile("ld.global.L1::no_allocate.L2::256B.v4.u32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+                 : "l"(p)
+                 : "memory");
+    return r;
+}
 __device__ __forceinline__ uint4 ldg_stream16(const void* p) {
     uint4 r;
     asm volatile("ld.global.nc.L1::no_allocate.L2::256B.v4.u32 {%0,%1,%2,%3}, [%4];"

@@ -166,7 +166,7 @@ k_reduce(const T* in, uint64_t n, uint64_t head, Xf xf, Op op, A ident, A* parti
     for (; i + (kUnroll - 1) * G < nv; i += kUnroll * G) {
         uint4 r[kUnroll];
 #pragma unroll
-        for (int u = 0; u < kUnroll; ++u) r[u] = ldg_stream16(vp + i + u * G);
+        for (int u = 0; u < kUnroll; ++u) r[u] = ld_stream16(vp + i + u * G);
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u) {
             const T* e = reinterpret_cast<const T*>(&r[u]);
@@ -176,7 +176,7 @@ k_reduce(const T* in, uint64_t n, uint64_t head, Xf xf, Op op, A ident, A* parti
         }
     }
     for (; i < nv; i += G) {
-        uint4 r = ldg_stream16(vp + i);
+        uint4 r = ld_stream16(vp + i);
         const T* e = reinterpret_cast<const T*>(&r);
         const uint64_t base = head + i * V;
 #pragma unroll

@@ -219,7 +219,7 @@ __device__ __forceinline__ ItemDesc load_desc(const ItemDesc* items, uint32_t i)
     const uint4* p = reinterpret_cast<const uint4*>(items + i);
     uint4 w[3];
 #pragma unroll
-    for (int q = 0; q < 3; ++q) w[q] = __ldg(p + q);
+    for (int q = 0; q < 3; ++q) w[q] = p[q];
     ItemDesc d;
     memcpy(&d, w, sizeof d);
     return d;
@@ -463,7 +463,7 @@ k_segmented(SegArgs<T> a, SegBuffers b, volatile int32_t* err) {
                 const int j = q * BLOCK + tid;
                 const int e0 = j * V - (int)mis;
                 v[q] = vec_ok && e0 >= 0 && e0 + V <= (int)len
-                           ? ldg_stream16(base + j * V)
+                           ? ld_stream16(base + j * V)
                            : make_uint4(0u, 0u, 0u, 0u);
             }
             auto fold = [&](auto red_c) {

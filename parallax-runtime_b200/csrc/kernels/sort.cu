@@ -164,8 +164,8 @@ __device__ __forceinline__ Pair pair_of(uint64_t o, uint64_t n, uint64_t L) {
 // of the stable merge of A[0, la) and B[0, lb) (A wins ties): the number of i < d with
 // B[d-1-i] >= A[i] (a monotone predicate), found by a 32-ary search (32 probes a round).
 template <typename K>
-__device__ __forceinline__ uint64_t warp_merge_split(const K* __restrict__ A, uint64_t la,
-                                                     const K* __restrict__ B, uint64_t lb,
+__device__ __forceinline__ uint64_t warp_merge_split(const K* A, uint64_t la,
+                                                     const K* B, uint64_t lb,
                                                      uint64_t d) {
     const int lane = threadIdx.x & 31;
     uint64_t lo = d > lb ? d - lb : 0;
@@ -215,7 +215,7 @@ constexpr int staged_elems(int ot) { return ot + 2 * SortShape<K>::ITEMS + 4 * (
 // output), then stores them as 16-byte vectors (a thread's outputs are contiguous).
 template <typename K, int XF>
 __device__ __forceinline__ void merge_spans(const K* As, int na, const K* Bs, int nb,
-                                            K* __restrict__ dst, bool final_pass) {
+                                            K* dst, bool final_pass) {
     constexpr int IPT = SortShape<K>::ITEMS;
     constexpr int V = 16 / sizeof(K);
     const int total = na + nb;
@@ -318,8 +318,8 @@ __device__ __forceinline__ void stage_store(K* sm, int na, int nb, const SpanPla
 // aligned 16-byte loads, all of a thread's vectors of both spans in flight at once, then
 // merges them.
 template <typename K, int XF>
-__device__ __forceinline__ void merge_tile(const K* __restrict__ A, int na, const K* __restrict__ B,
-                                           int nb, K* __restrict__ dst, bool final_pass, K* sm) {
+__device__ __forceinline__ void merge_tile(const K* A, int na, const K* B,
+                                           int nb, K* dst, bool final_pass, K* sm) {
     const SpanPlace q = span_place(A, na, B, nb);
     uint4 r[stage_vectors<K>()];
     stage_load(A, B, q, r);

@@ -5,9 +5,10 @@
 // still runs. It calls dependent_prologue() before its first access to global memory: that
 // lets its own successor start early and then waits until the predecessor has finished and
 // its writes are visible. Every kernel of a chain waits, so the order of the whole chain
-// holds. Before the call a kernel may only touch its parameters and shared memory. Its pointers to
-// data of earlier kernels are not __restrict__: a load the compiler takes for invariant could be
-// moved above the wait.
+// holds. Before the call a kernel may only touch its parameters and shared memory. It reads
+// global memory with coherent loads only: no __ldg, no ld.global.nc, no __restrict__ pointer. A
+// read-only load wants data that nothing writes during the kernel's lifetime, which here begins
+// while earlier kernels still write, and the compiler may move it above the wait.
 // Measured on B200: a radix sort of 100,003 int64 keys (nine launches) 93 -> 70 us, of 2^20
 // uint32 keys (five) 71 -> 60 us.
 #pragma once

@@ -50,7 +50,7 @@ struct PredDev {
                     const uint32_t* w = reinterpret_cast<const uint32_t*>(fl + gi);
 #pragma unroll
                     for (int v = 0; v < ITEMS / 4; ++v) {
-                        const uint32_t b = __ldg(w + v);
+                        const uint32_t b = w[v];
 #pragma unroll
                         for (int k = 0; k < 4; ++k)
                             if ((b >> (8 * k)) & 0xffu) f |= 1u << (4 * v + k);
@@ -60,7 +60,7 @@ struct PredDev {
                     const uint16_t* w = reinterpret_cast<const uint16_t*>(fl + gi);
 #pragma unroll
                     for (int v = 0; v < ITEMS / 2; ++v) {
-                        const uint32_t b = __ldg(w + v);
+                        const uint32_t b = w[v];
 #pragma unroll
                         for (int k = 0; k < 2; ++k)
                             if ((b >> (8 * k)) & 0xffu) f |= 1u << (2 * v + k);

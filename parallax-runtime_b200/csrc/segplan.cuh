@@ -38,10 +38,10 @@ struct SegSrc {
     uint32_t elem;            // element bytes
 
     __device__ __forceinline__ uint64_t begin(uint64_t s) const {
-        return offsets ? __ldg(&offsets[s]) : 0;
+        return offsets ? offsets[s] : 0;
     }
     __device__ __forceinline__ uint64_t len(uint64_t s) const {
-        return offsets ? __ldg(&offsets[s + 1]) - __ldg(&offsets[s]) : descs[s].n;
+        return offsets ? offsets[s + 1] - offsets[s] : descs[s].n;
     }
     __device__ __forceinline__ uint64_t in_addr(uint64_t s) const {
         return offsets ? in + begin(s) * elem : descs[s].in;
@@ -62,7 +62,7 @@ __device__ __forceinline__ uint32_t find_segment(const uint32_t* item_start, uin
     uint64_t lo = 0, hi = S;
     while (hi - lo > 1) {
         const uint64_t mid = (lo + hi) >> 1;
-        if (__ldg(&item_start[mid]) <= item) lo = mid;
+        if (item_start[mid] <= item) lo = mid;
         else hi = mid;
     }
     return (uint32_t)lo;
