@@ -422,6 +422,7 @@ k_compact_pipe(const T* in, T* out, uint64_t n, uint32_t num_tiles, PredDev<T> p
             wait_bar(&published[b], phase(it), ts.err);
             const uint64_t kept = s_kept[b];
             const uint64_t prefix = lookback_warp<uint64_t>(ts, t, kept);
+            __syncwarp();  // every lane has read the slot (the first tile's walk has no step)
             if (lane == 0) {
                 s_prefix[b] = prefix;
                 if (t == num_tiles - 1) *count_out = MODE == 2 ? *num_true : prefix + kept;

@@ -1186,6 +1186,7 @@ k_seg_select_pipe(SegArgs<T> a, PredDev<T> pred, SegBuffers b, volatile int32_t*
             wait_bar(&published[s], phase(it), err);
             const uint64_t kept = s_kept[s];
             const uint64_t prefix = lookback_warp<uint64_t>(ts, item, kept, s_it[s].first);
+            __syncwarp();  // every lane has read the slot (a first item's walk has no step)
             if (lane == 0) {
                 s_prefix[s] = prefix;
                 if (s_it[s].last) *reinterpret_cast<uint64_t*>(s_it[s].aux) = prefix + kept;

@@ -2,7 +2,11 @@
 results only when the timing is unlucky.
 
 * Kernels launched as dependents (pdl.cuh) start while earlier kernels of their stream still write, so
-  they and their device functions use no read-only load: no __ldg, ld.global.nc or __restrict__."""
+  they and their device functions use no read-only load: no __ldg, ld.global.nc or __restrict__.
+* In the pipelines one lane arrives for its warp on the barrier that lets other warps, and in the end the
+  mover, write to a buffer and its slot. Between the wait that gave the warp the slot and the arrival the
+  whole warp meets (__syncwarp, or a warp reduction that every lane takes part in), so that no lane still
+  reads the slot."""
 from __future__ import annotations
 
 import re
@@ -33,3 +37,19 @@ def test_dependent_kernels_use_no_read_only_loads():
             if bad and not plain and " ldg_stream16(const void* p) {" not in fn:
                 raise AssertionError((f.name, bad, fn[:200]))
     assert kernels > 15  # the dependent kernels were found
+
+
+def test_warps_meet_before_a_lane_arrives_for_them():
+    arrivals = 0
+    for f in files():
+        for fn in functions(f.read_text()):
+            if not fn.startswith("__global__"):
+                continue
+            for m in re.finditer(r"mbar_arrive\(&(\w+)\[", fn):
+                if m.group(1) == "full":  # the mover, a single lane
+                    continue
+                arrivals += 1
+                waits = [w.end() for w in re.finditer(r"\bwait_bar\(|\blanded\(", fn[:m.start()])]
+                since = fn[waits[-1]:m.start()]
+                assert "__syncwarp();" in since or "__reduce_add_sync(" in since, (f.name, m.group(0), since)
+    assert arrivals >= 15
