@@ -6,12 +6,13 @@
 // shaders/scan_add.comp:14-19); exclusive adds a shift pass writing
 // out[i] = init + incl[i-1] (kernel_launcher.cpp:1346-1475).
 //
-// Here: one launch. 16-byte-aligned device operands go through a persistent pipeline, one
-// warp-specialised CTA per SM (k_scan_pipe): tiles are bulk-loaded (cp.async.bulk) into a ring of
-// buffers, summed and published as they land, looked back (lookback.cuh) while later tiles load,
-// scanned in place and bulk-stored. Operands that are not aligned or lie in the host mirror, scans
-// whose copies overlap their tiles, and the allocation-free entry point take one 512-thread CTA
-// per 112 KiB tile (two per SM), in blockIdx order (k_scan): stage, sum, look back, rescan, store.
+// Here: one launch. 16-byte-aligned device operands of more than a wave of tiles go through a
+// persistent pipeline, one warp-specialised CTA per SM (k_scan_pipe): tiles are bulk-loaded
+// (cp.async.bulk) into a ring of buffers, summed and published as they land, looked back
+// (lookback.cuh) while later tiles load, scanned in place and bulk-stored. Smaller ones, operands
+// that are not aligned or lie in the host mirror, scans whose copies overlap their tiles, and the
+// allocation-free entry point take one 512-thread CTA per 112 KiB (smallest arrays: 56 KiB) tile
+// (two per SM), in blockIdx order (k_scan): stage, sum, look back, rescan, store.
 // Rows are 28 (4-byte) or 14 (8-byte) consecutive elements per thread (112 bytes, an odd number
 // of 16-byte words: conflict-free 128-bit shared loads).
 // HBM traffic is the algorithmic minimum: n*s read + n*s written.
@@ -261,14 +262,15 @@ k_scan_pipe(const T* in, T* out, uint64_t n, uint32_t num_tiles,
     constexpr int V = PipeShape<T>::V, ITEMS = PipeShape<T>::ITEMS, TILE = PipeShape<T>::TILE;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     T* const bufs = reinterpret_cast<T*>(smem_raw);
-    __shared__ __align__(8) uint64_t full[kPipeStages], summed[kPipeStages], ready[kPipeStages],
-        written[kPipeStages];
+    __shared__ __align__(8) uint64_t full[kPipeStages], added[kPipeStages], summed[kPipeStages],
+        ready[kPipeStages], written[kPipeStages];
     __shared__ A s_tot[kPipeStages][kPipeWarps], s_off[kPipeStages][kPipeWarps], s_agg[kPipeStages];
     __shared__ uint32_t s_tile[kPipeStages];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
         for (int s = 0; s < kPipeStages; ++s) {
             mbar_init(&full[s], 1);
+            mbar_init(&added[s], kSumWarps);
             mbar_init(&summed[s], 1);
             mbar_init(&ready[s], 1);
             mbar_init(&written[s], kPipeWarps);
@@ -348,8 +350,10 @@ k_scan_pipe(const T* in, T* out, uint64_t n, uint32_t num_tiles,
                 const A tot = warp_reduce((A)sum, OpSum());
                 if (lane == 0) s_tot[b][part] = tot;
             }
-            asm volatile("bar.sync 1, %0;" ::"n"(kSumWarps * 32) : "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&added[b]);
             if (sw == 0) {
+                wait_bar(&added[b], ph, ts.err);
                 const A v = lane < kPipeWarps ? s_tot[b][lane] : A(0);
                 const A vi = warp_inclusive_scan(v, OpSum());
                 const A agg = shfl_idx(vi, 31);

@@ -806,14 +806,15 @@ k_seg_scan_pipe(SegArgs<T> a, SegBuffers b, volatile int32_t* err) {
     constexpr int V = Sh::V, ITEMS = Sh::ITEMS, PART = Sh::PART, SLOTS = Sh::SLOTS;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     T* const bufs = reinterpret_cast<T*>(smem_raw);
-    __shared__ __align__(8) uint64_t full[kPipeStages], summed[kPipeStages], ready[kPipeStages],
-        written[kPipeStages];
+    __shared__ __align__(8) uint64_t full[kPipeStages], added[kPipeStages], summed[kPipeStages],
+        ready[kPipeStages], written[kPipeStages];
     __shared__ A s_tot[kPipeStages][kScanWarps], s_off[kPipeStages][kScanWarps], s_agg[kPipeStages];
     __shared__ PipeItem<T> s_it[kPipeStages];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
         for (int s = 0; s < kPipeStages; ++s) {
             mbar_init(&full[s], 1);
+            mbar_init(&added[s], kSumWarps);
             mbar_init(&summed[s], 1);
             mbar_init(&ready[s], 1);
             mbar_init(&written[s], kScanWarps);
@@ -912,8 +913,10 @@ k_seg_scan_pipe(SegArgs<T> a, SegBuffers b, volatile int32_t* err) {
                 const A tot = warp_reduce((A)sum, OpSum());
                 if (lane == 0) s_tot[s][part] = tot;
             }
-            asm volatile("bar.sync 1, %0;" ::"n"(kSumWarps * 32) : "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&added[s]);
             if (sw == 0) {
+                wait_bar(&added[s], phase(it), err);
                 const A v = lane < kScanWarps ? s_tot[s][lane] : A(0);
                 const A vi = warp_inclusive_scan(v, OpSum());
                 const A agg = shfl_idx(vi, 31);

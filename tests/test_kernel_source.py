@@ -6,7 +6,9 @@ results only when the timing is unlucky.
 * In the pipelines one lane arrives for its warp on the barrier that lets other warps, and in the end the
   mover, write to a buffer and its slot. Between the wait that gave the warp the slot and the arrival the
   whole warp meets (__syncwarp, or a warp reduction that every lane takes part in), so that no lane still
-  reads the slot."""
+  reads the slot.
+* Every wait between warps ends by itself: they meet at an mbarrier, polled up to a limit (wait_bar), not
+  at a named barrier, which waits forever for a warp that gave up another wait."""
 from __future__ import annotations
 
 import re
@@ -53,3 +55,8 @@ def test_warps_meet_before_a_lane_arrives_for_them():
                 since = fn[waits[-1]:m.start()]
                 assert "__syncwarp();" in since or "__reduce_add_sync(" in since, (f.name, m.group(0), since)
     assert arrivals >= 15
+
+
+def test_no_unbounded_named_barriers():
+    for f in files():
+        assert not re.search(r"\bbar\.sync\b|\bbarrier\.sync\b|\bbarrier\.cta\.sync\b", f.read_text()), f.name
