@@ -1362,10 +1362,17 @@ uint64_t shape_tile(const SegCall& c, int shape) {
         return es == 4 ? pipe_tile<uint32_t>(c.op) : pipe_tile<uint64_t>(c.op);
     return (uint64_t)kShapes[shape].block * kShapes[shape].vpt * V - V;
 }
-// Whether the pipeline takes the call: a scan or a select by predicate of one element-aligned array.
+// Whether an array can be bulk-loaded item by item: one element-aligned array in HBM. (Operands in
+// the page-locked host mirror, which whole-heap capture uses in place, take plain loads here as in
+// the plain scans and compactions.)
+bool bulk_input(const SegCall& c) {
+    return c.src.offsets && c.src.in % dtype_size(c.t) == 0 &&
+           !arena_contains(reinterpret_cast<const void*>(c.src.in));
+}
+// Whether the pipeline takes the call: a scan or a select by predicate.
 bool pipe_takes(const SegCall& c) {
-    return (c.op == SEG_SCAN || (c.op == SEG_SELECT && !c.unique)) && c.src.offsets &&
-           c.src.in % dtype_size(c.t) == 0 && c.src.out % dtype_size(c.t) == 0;
+    return (c.op == SEG_SCAN || (c.op == SEG_SELECT && !c.unique)) && bulk_input(c) &&
+           c.src.out % dtype_size(c.t) == 0;
 }
 
 template <typename T>
@@ -1393,10 +1400,13 @@ bool enqueue_pipe(Workspace& ws, const SegCall& c, const SegBuffers& b) {
                             "segmented select launch", args, make_pred<T>(c.pred), b, err);
 }
 
-// Whether a reduce of the {512, 7} shape runs as the pipeline: sums and extremes of one
-// element-aligned array.
+// Whether a reduce of the {512, 7} shape runs as the pipeline: sums and extremes.
 bool reduce_pipe_takes(const SegCall& c) {
-    return c.op == SEG_REDUCE && c.red != RED_COUNT && c.src.offsets && c.src.in % dtype_size(c.t) == 0;
+    return c.op == SEG_REDUCE && c.red != RED_COUNT && bulk_input(c);
+}
+// Whether the call with this shape runs as a pipeline.
+bool runs_pipe(const SegCall& c, int shape) {
+    return shape == kPipeShape || (shape == 2 && reduce_pipe_takes(c));
 }
 
 template <typename T, int RED>
@@ -1526,8 +1536,9 @@ int tuned_shape(Workspace& ws, const SegCall& c) {
         float ms = 0;
         cudaEventElapsedTime(&ms, e0, e1);
         if (getenv("PARALLAX_DEBUG"))
-            fprintf(stderr, "[parallax] segmented op %d dtype %d bucket %d: %d threads x %d vectors %.3f ms\n",
-                    opkey, (int)c.t, bucket_of(c), kShapes[cand].block, kShapes[cand].vpt, ms);
+            fprintf(stderr, "[parallax] segmented op %d dtype %d bucket %d: %d threads x %d vectors%s %.3f ms\n",
+                    opkey, (int)c.t, bucket_of(c), kShapes[cand].block, kShapes[cand].vpt,
+                    runs_pipe(c, cand) ? " (pipeline)" : "", ms);
         if (ms < best_ms) {
             best_ms = ms;
             best = cand;
