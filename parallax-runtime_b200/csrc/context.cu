@@ -126,9 +126,9 @@ Workspace* new_workspace() {
     return ws;
 }
 
-// Bytes of one look-back status entry (lookback.cuh): {u32 flag, u32 pad, u64 agg,
-// u64 inc} for every accumulator type, so flag words sit at the same addresses in every
-// launch.
+// Bytes of one look-back status entry (lookback.cuh): {u32 low value bits, u32 flag, u32 high
+// value bits, u32 flag} for every accumulator type, so flag words sit at the same addresses in
+// every launch.
 static constexpr size_t kStatusEntry = sizeof(StatusEntry);
 
 // Replaces a workspace buffer by a larger one (at least `bytes`, doubling from `min_cap`),
@@ -173,9 +173,17 @@ char* Workspace::scratch(uint64_t tiles) {
     return static_cast<char*>(d_scratch);
 }
 
+// The launch epoch lies in this buffer and starts again when it is replaced: the look-back entries of
+// earlier launches, in a buffer of their own, are cleared with it.
 void* Workspace::seg(size_t bytes) {
     if (bytes <= seg_cap) return d_seg;
-    return regrow(*this, &d_seg, &seg_cap, bytes, 1 << 20, true, "segment buffer") ? d_seg : nullptr;
+    if (!regrow(*this, &d_seg, &seg_cap, bytes, 1 << 20, true, "segment buffer")) return nullptr;
+    if (d_seg_status && !cuda_ok(cudaMemsetAsync(d_seg_status, 0, seg_status_cap * kStatusEntry, stream()),
+                                 "segment status clear")) {
+        seg_cap = 0;  // not usable with the old entries: replaced again by the next call
+        return nullptr;
+    }
+    return d_seg;
 }
 
 void* Workspace::seg_status(uint64_t entries) {
