@@ -131,6 +131,23 @@ Workspace* new_workspace() {
 // every launch.
 static constexpr size_t kStatusEntry = sizeof(StatusEntry);
 
+// First sizes of the buffers that hold spread look-back entries (lookback.cuh): what the same call of
+// packed entries would fit into 1 MiB (plain: 2^17 tiles, some 7 GB of data) or 256 KiB (segmented:
+// 2^14 work items). A call that outgrows its buffer is refused inside a stream capture, and a
+// replaced buffer is gone for graphs that a program captured before, so this does not come earlier
+// because entries lie apart. The segmented radix sort's small batches have smaller tiles, at most
+// one more for every SM.
+static constexpr size_t kScratchMin = kScratchSmall + ((size_t(1) << 17) << kStatusLineShift) * kStatusEntry;
+static constexpr size_t kSegStatusMin = ((size_t(1) << 14) << kStatusLineShift) * kStatusEntry;
+static constexpr size_t kSegRadixMin = 2 << 20;
+
+bool stream_capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    const bool yes = cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return yes;
+}
+
 // Replaces a workspace buffer by a larger one (at least `bytes`, doubling from `min_cap`),
 // optionally zeroed. In stream order: cudaFreeAsync / cudaMallocAsync on the workspace's
 // stream wait only for that stream's earlier work (which may still use the old buffer),
@@ -140,12 +157,10 @@ static constexpr size_t kStatusEntry = sizeof(StatusEntry);
 static bool regrow(Workspace& ws, void** buf, size_t* cap_io, size_t bytes, size_t min_cap,
                    bool zero, const char* what) {
     cudaStream_t s = ws.stream();
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) {
+    if (stream_capturing(s)) {
         set_error(PARALLAX_ERR_INVALID_ARGUMENT, "%s: buffer growth inside a stream capture", what);
         return false;
     }
-    cudaGetLastError();
     if (*buf) {
         if (!cuda_ok(cudaFreeAsync(*buf, s), what)) return false;
         *buf = nullptr;
@@ -168,7 +183,7 @@ char* Workspace::scratch(uint64_t tiles) {
     if (bytes <= scratch_cap) return static_cast<char*>(d_scratch);
     // Zeroed: look-back status words then read as "not ready" for every epoch, and the
     // self-resetting ticket counters start at zero.
-    if (!regrow(*this, &d_scratch, &scratch_cap, bytes, 1 << 20, true, "scratch")) return nullptr;
+    if (!regrow(*this, &d_scratch, &scratch_cap, bytes, kScratchMin, true, "scratch")) return nullptr;
     epoch = 1;
     return static_cast<char*>(d_scratch);
 }
@@ -189,8 +204,8 @@ void* Workspace::seg(size_t bytes) {
 void* Workspace::seg_status(uint64_t entries) {
     if (entries <= seg_status_cap) return d_seg_status;
     size_t bytes_cap = seg_status_cap * kStatusEntry;
-    if (!regrow(*this, &d_seg_status, &bytes_cap, entries * kStatusEntry, (1 << 14) * kStatusEntry,
-                true, "segment status"))
+    if (!regrow(*this, &d_seg_status, &bytes_cap, entries * kStatusEntry, kSegStatusMin, true,
+                "segment status"))
         return nullptr;
     seg_status_cap = bytes_cap / kStatusEntry;
     return d_seg_status;
@@ -205,7 +220,7 @@ void* Workspace::radix(size_t bytes) {
 
 void* Workspace::seg_radix(size_t bytes) {
     if (bytes <= seg_radix_cap) return d_seg_radix;
-    return regrow(*this, &d_seg_radix, &seg_radix_cap, bytes, 1 << 20, true,
+    return regrow(*this, &d_seg_radix, &seg_radix_cap, bytes, kSegRadixMin, true,
                   "segmented radix buffer")
                ? d_seg_radix
                : nullptr;

@@ -709,6 +709,18 @@ bool seg_radix_sort_keys(Workspace& ws, SegSrc src, uint64_t count, uint64_t S, 
     return graph_launch(ws, key, enqueue);
 }
 
+// The radix buffer: [0, 256) tile claim / exit counters, then a histogram per digit position, then
+// the per-(tile, digit) look-back words.
+constexpr size_t kRadixHistOff = 256;
+template <typename K>
+constexpr size_t kRadixStatusOff = kRadixHistOff + sizeof(K) * kBins * 8;
+
+template <typename K>
+size_t radix_bytes(uint64_t n) {
+    const uint64_t tile = (uint64_t)RadixShape<K>::BLOCK * radix_rows<K>(n);
+    return kRadixStatusOff<K> + (n + tile - 1) / tile * kBins * 8;
+}
+
 // Digit passes p0 .. P-1: p0 = 0 sorts by the whole key; p0 = 4 on 8-byte records sorts
 // them stably by their high 32 bits alone (LSD passes are stable), the (key << 32 | value)
 // records of a sort_kv handle.
@@ -725,15 +737,12 @@ bool radix_sort_keys(Workspace& ws, void* d_data, uint64_t n, int p0 = 0) {
     K* data = static_cast<K*>(d_data);
     K* tmp = static_cast<K*>(ws.temp(n * sizeof(K)));
     if (!tmp) return false;
-    // radix buffer: [0, 256) tile claim / exit counters, then P histograms, then the
-    // per-(tile, digit) look-back words
-    constexpr size_t hist_off = 256, status_off = hist_off + (size_t)P * kBins * 8;
-    char* rb = static_cast<char*>(ws.radix(status_off + tiles * kBins * 8));
+    char* rb = static_cast<char*>(ws.radix(radix_bytes<K>(n)));
     if (!rb) return false;
     const uint32_t ep0 = ws.next_radix_epochs(P);
     uint32_t* counters = reinterpret_cast<uint32_t*>(rb);
-    auto* hist = reinterpret_cast<unsigned long long*>(rb + hist_off);
-    auto* status = reinterpret_cast<uint64_t*>(rb + status_off);
+    auto* hist = reinterpret_cast<unsigned long long*>(rb + kRadixHistOff);
+    auto* status = reinterpret_cast<uint64_t*>(rb + kRadixStatusOff<K>);
     volatile int32_t* err = &ws.d_slot->spin_error;
     cudaStream_t s = ws.stream();
     if (!cuda_ok(cudaMemsetAsync(hist, 0, (size_t)P * kBins * 8, s), "radix histogram clear"))
@@ -804,6 +813,10 @@ bool launch_segmented_radix_sort(Workspace& ws, DType t, const SegSrc& src, uint
 uint64_t segmented_radix_tile(DType t) {
     return dtype_size(t) == 4 ? (uint64_t)RadixShape<uint32_t>::BLOCK * RadixShape<uint32_t>::ITEMS
                               : (uint64_t)RadixShape<uint64_t>::BLOCK * RadixShape<uint64_t>::ITEMS;
+}
+
+size_t radix_buffer_bytes(DType t, size_t n) {
+    return dtype_size(t) == 4 ? radix_bytes<uint32_t>(n) : radix_bytes<uint64_t>(n);
 }
 
 bool launch_radix_sort(Workspace& ws, DType t, void* d_data, size_t n, bool by_key) {

@@ -650,6 +650,9 @@ bool launch_sort(Workspace& ws, DType t, void* d_data, size_t n, bool by_key) {
     if (by_key) return launch_radix_sort(ws, t, d_data, n, true);
     const size_t es = dtype_size(t);
     bool radix = n >= sort_radix_min(t);
+    // No buffer can grow inside a stream capture, and a program may have warmed up with smaller
+    // sorts: the merge sort does without the radix sort's buffer.
+    if (radix && ws.radix_cap < radix_buffer_bytes(t, n) && stream_capturing(ws.stream())) radix = false;
     if (const char* e = getenv("PARALLAX_SORT")) {
         if (!strcmp(e, "merge")) radix = false;
         else if (!strcmp(e, "radix")) radix = true;

@@ -160,6 +160,9 @@ Workspace* workspace();  // the calling thread's; nullptr when the device is una
 Workspace* current_workspace();  // the calling thread's if it has one, else nullptr
 Workspace* new_workspace();  // an independent one (own stream and buffers), never freed
 
+// Whether the stream is being captured, by the runtime or by the caller.
+bool stream_capturing(cudaStream_t s);
+
 // Replays the CUDA graph cached under `key` on the workspace stream, capturing it first
 // (thread-local capture of what `enqueue` puts on the stream) when it is missing or was
 // captured before a buffer reallocation. `enqueue` must not grow workspace buffers.
@@ -320,6 +323,8 @@ bool launch_sort(Workspace& ws, DType t, void* d_data, size_t n, bool by_key = f
 // Smallest array launch_sort gives to the radix sort (by default; PARALLAX_SORT overrides).
 size_t sort_radix_min(DType t);
 // One-sweep LSD radix sort (kernels/radix.cu); launch_sort picks it for large arrays.
+// radix_buffer_bytes: what it needs of Workspace::radix.
+size_t radix_buffer_bytes(DType t, size_t n);
 bool launch_radix_sort(Workspace& ws, DType t, void* d_data, size_t n, bool by_key = false);
 bool launch_map(Workspace& ws, MapOp op, const void* d_in, void* d_out, size_t n,
                 const void* captures, size_t capture_size);
