@@ -1463,9 +1463,16 @@ bool enqueue(Workspace& ws, const SegCall& c, int shape) {
 // ---- autotuner -----------------------------------------------------------------------------------
 // Shape per (op, dtype, log2 of the average segment length); timed on the first call with
 // those parameters, optionally persisted in PARALLAX_TUNE_CACHE, one line per choice:
-// "op dtype bucket block vpt".
+// "op dtype bucket block vpt". Calls that a pipeline takes have entries of their own (kPipeKey is
+// added to the op): the others, descriptor batches above all, choose among the tile kernels, and
+// neither's choice is forced on the other (512 x 7 is a pipeline for one and the slowest reduce for
+// the other). Timing a call of the first kind finds the entry of the second as well.
 std::mutex g_tune_mu;
 std::map<std::tuple<int, int, int>, int>* g_tune = nullptr;
+
+constexpr int kPipeKey = 64;
+int op_key(const SegCall& c) { return c.op * 8 + c.red * 2 + (c.unique ? 1 : 0); }
+bool takes_pipe(const SegCall& c) { return pipe_takes(c) || reduce_pipe_takes(c); }
 
 int shape_index(int block, int vpt) {
     for (int i = 0; i < kNumShapes; ++i)
@@ -1481,10 +1488,16 @@ void tune_load_locked() {
     FILE* f = fopen(path, "r");
     if (!f) return;
     int op, t, bucket, block, vpt;
+    std::map<std::tuple<int, int, int>, int> shared;  // of files without the pipelines' own entries
     while (fscanf(f, "%d %d %d %d %d", &op, &t, &bucket, &block, &vpt) == 5) {
         const int i = shape_index(block, vpt);
-        if (i >= 0) (*g_tune)[std::make_tuple(op, t, bucket)] = i;
+        if (i < 0) continue;
+        if (op >= kPipeKey || i != kPipeShape) (*g_tune)[std::make_tuple(op, t, bucket)] = i;
+        const bool has_pipe = op == SEG_SCAN * 8 || op == SEG_SELECT * 8 ||
+                              (op >= 0 && op <= RED_MIN * 2 && op % 2 == 0);
+        if (has_pipe) shared[std::make_tuple(op + kPipeKey, t, bucket)] = i;
     }
+    g_tune->insert(shared.begin(), shared.end());
     fclose(f);
 }
 
@@ -1508,23 +1521,27 @@ int bucket_of(const SegCall& c) {
 
 // Returns the shape choice, timing the candidates (and leaving valid results) when unknown.
 int tuned_shape(Workspace& ws, const SegCall& c) {
-    const int opkey = c.op * 8 + c.red * 2 + (c.unique ? 1 : 0);
-    const auto key = std::make_tuple(opkey, (int)c.t, bucket_of(c));
+    const int opkey = op_key(c);
+    const bool pipe = takes_pipe(c);
+    const bool may_time = c.tune && !(getenv("PARALLAX_TUNE") && atoi(getenv("PARALLAX_TUNE")) == 0);
+    const auto tile_key = std::make_tuple(opkey, (int)c.t, bucket_of(c));
+    const auto key = std::make_tuple(opkey + (pipe ? kPipeKey : 0), (int)c.t, bucket_of(c));
     {
         std::lock_guard<std::mutex> g(g_tune_mu);
         tune_load_locked();
         auto it = g_tune->find(key);
+        if (it == g_tune->end() && !may_time) it = g_tune->find(tile_key);
         if (it != g_tune->end() && (it->second != kPipeShape || pipe_takes(c))) return it->second;
     }
-    if (!c.tune || (getenv("PARALLAX_TUNE") && atoi(getenv("PARALLAX_TUNE")) == 0)) {
+    if (!may_time) {
         const uint64_t avg = c.S ? c.count / c.S : 0;  // untuned: by average segment length
         return avg >= (16u << 10) ? 2 : avg >= (2u << 10) ? 1 : 0;
     }
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    int best = 1;
-    float best_ms = 1e30f;
+    int best = 1, best_tile = 1;
+    float best_ms = 1e30f, best_tile_ms = 1e30f;
     cudaStream_t s = ws.stream();
     for (int cand = 0; cand < kNumShapes; ++cand) {
         if (cand == kPipeShape && !pipe_takes(c)) continue;
@@ -1543,11 +1560,16 @@ int tuned_shape(Workspace& ws, const SegCall& c) {
             best_ms = ms;
             best = cand;
         }
+        if (ms < best_tile_ms && !runs_pipe(c, cand)) {
+            best_tile_ms = ms;
+            best_tile = cand;
+        }
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     std::lock_guard<std::mutex> g(g_tune_mu);
     (*g_tune)[key] = best;
+    if (pipe) g_tune->emplace(tile_key, best_tile);
     tune_store_locked();
     if (getenv("PARALLAX_DEBUG"))
         fprintf(stderr,
