@@ -1534,8 +1534,15 @@ int tuned_shape(Workspace& ws, const SegCall& c) {
         if (it != g_tune->end() && (it->second != kPipeShape || pipe_takes(c))) return it->second;
     }
     if (!may_time) {
-        const uint64_t avg = c.S ? c.count / c.S : 0;  // untuned: by average segment length
-        return avg >= (16u << 10) ? 2 : avg >= (2u << 10) ? 1 : 0;
+        // Not timed: by mean length. The scan and select pipelines win from some 6 K elements (60 M
+        // elements in all, us, pipeline / 256 x 7: lognormal segments of mean 6 K fp32 scan 216 / 243,
+        // copy_if 210 / 329, equal ones of 8 K int32 165 / 269 and 183 / 464; mean 3 K, fp32 scan: 370 /
+        // 316). As a tile kernel 512 x 7 never does (mean 24 K, fp32, 512 x 7 / 256 x 7: scan 325 / 196,
+        // select 286 / 241, partition 390 / 326, unique 249 / 210; reduces 149 / 121 at mean 30 K).
+        const uint64_t avg = c.S ? c.count / c.S : 0;
+        if (pipe && avg >= (c.op == SEG_REDUCE ? 16u << 10 : 8u << 10))
+            return c.op == SEG_REDUCE ? 2 : kPipeShape;
+        return avg >= (2u << 10) ? 1 : 0;
     }
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
