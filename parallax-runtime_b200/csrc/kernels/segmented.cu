@@ -1780,7 +1780,7 @@ int seg_compact_entry(parallax_kernel_t kernel, const void* input, void* output,
     c.t = h->dtype;
     c.count = count;
     c.S = num_segments;
-    c.tune = which != 1 || input != output;
+    c.tune = input != output;  // timed in place, a run would compact what the one before has left
     c.pred = h->pred;
     if (h->kind == Kind::COMPACT_FLAGS && h->remove) c.pred.negate = !c.pred.negate;
     return seg_entry(c, input, output, offsets, counts, fn);
