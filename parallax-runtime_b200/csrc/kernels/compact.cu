@@ -189,22 +189,21 @@ __device__ __forceinline__ void compact_tile(T* buf, uint64_t* bars, uint32_t pa
     __syncthreads();  // buffer and shared state free for the next tile
 }
 
-// One CTA per tile of NSUB sub-tiles (arrays of at most a wave, unaligned inputs), in blockIdx order, or in the order of an atomic claim counter when
-// `claim` is given (see tile_claim()).
+// One CTA per tile of NSUB sub-tiles (arrays of at most a wave, unaligned inputs), in blockIdx order
+// (see k_scan).
 template <typename T, int MODE, bool BULK, int NSUB>
 __global__ void __launch_bounds__(kBlock, kCtasPerSm)
 k_compact(const T* in, T* out, uint64_t n, PredDev<T> pred, TileStatus<uint64_t> ts,
           const unsigned long long* num_true,
-          unsigned long long* count_out, uint32_t* claim) {
+          unsigned long long* count_out) {
     constexpr int SUB = Shape<T>::SUB;
     constexpr int TILE = NSUB * SUB;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     T* buf = reinterpret_cast<T*>(smem_raw);
     __shared__ __align__(8) uint64_t bars[NSUB];
     __shared__ CompactSmem sm;
-    __shared__ uint32_t s_claim;
     dependent_prologue();
-    const uint64_t tile = claim ? tile_claim(claim, s_claim) : blockIdx.x;
+    const uint64_t tile = blockIdx.x;
     const uint64_t base = tile * (uint64_t)TILE;
     const uint64_t rem = n - base;
     const uint32_t cnt = rem < (uint64_t)TILE ? (uint32_t)rem : (uint32_t)TILE;
@@ -213,7 +212,6 @@ k_compact(const T* in, T* out, uint64_t n, PredDev<T> pred, TileStatus<uint64_t>
     __syncthreads();
     compact_tile<T, MODE, BULK, NSUB>(buf, bars, 0, sm, tile, base, cnt, prev, out, n, pred, ts,
                                 num_true, count_out, tile == gridDim.x - 1);
-    if (claim && threadIdx.x == 0) persistent_exit(claim);
 }
 
 // Persistent pipeline without CTA-wide barriers, one CTA per SM (compare k_scan_pipe, scan.cu).
@@ -464,14 +462,13 @@ k_compact_pipe(const T* in, T* out, uint64_t n, uint32_t num_tiles, PredDev<T> p
 template <typename T, int MODE, bool BULK, int NSUB>
 bool launch_tiles(uint64_t n, cudaStream_t s, const T* in, T* out, PredDev<T> p,
                   TileStatus<uint64_t> ts, const unsigned long long* nt,
-                  unsigned long long* count_out, uint32_t* counters) {
+                  unsigned long long* count_out) {
     constexpr size_t smem = (size_t)NSUB * Shape<T>::SUB * sizeof(T);
     constexpr uint64_t tile = (uint64_t)NSUB * Shape<T>::SUB;
     if (!smem_opt_in<k_compact<T, MODE, BULK, NSUB>>(smem))
         return cuda_ok(cudaGetLastError(), "k_compact shared-memory opt-in");
     return launch_dependent(k_compact<T, MODE, BULK, NSUB>, (unsigned)((n + tile - 1) / tile), kBlock, smem,
-                            s, "k_compact launch", in, out, n, p, ts, nt, count_out,
-                            PXB_TILE_CLAIM ? counters : nullptr);
+                            s, "k_compact launch", in, out, n, p, ts, nt, count_out);
 }
 
 // Picks the kernel by size (in 112 KiB tiles), as the scans do: up to half a tile per SM single 56
@@ -481,11 +478,11 @@ bool launch_mode(uint64_t tiles, cudaStream_t s, bool bulk, const T* in, T* out,
                  PredDev<T> p, TileStatus<uint64_t> ts, const unsigned long long* nt,
                  unsigned long long* count_out, uint32_t* counters) {
     const uint64_t sms = device_info().sm_count;
-    if (!bulk) return launch_tiles<T, MODE, false, kSub>(n, s, in, out, p, ts, nt, count_out, counters);
+    if (!bulk) return launch_tiles<T, MODE, false, kSub>(n, s, in, out, p, ts, nt, count_out);
     if (tiles <= sms / 2)
-        return launch_tiles<T, MODE, true, 1>(n, s, in, out, p, ts, nt, count_out, counters);
+        return launch_tiles<T, MODE, true, 1>(n, s, in, out, p, ts, nt, count_out);
     if (tiles <= 2 * sms)
-        return launch_tiles<T, MODE, true, kSub>(n, s, in, out, p, ts, nt, count_out, counters);
+        return launch_tiles<T, MODE, true, kSub>(n, s, in, out, p, ts, nt, count_out);
     constexpr size_t smem = PipeShape<T>::SMEM;
     if (!smem_opt_in<k_compact_pipe<T, MODE>>(smem))
         return cuda_ok(cudaGetLastError(), "k_compact_pipe shared-memory opt-in");

@@ -190,13 +190,13 @@ __device__ __forceinline__ void scan_tile(T* buf, uint64_t* bars, uint32_t parit
 // `tile0` is the first tile of this launch: a scan launched in chunks (so its copies can
 // overlap its tiles) passes each chunk's first tile, and every chunk shares one look-back
 // epoch, so the first tile of a chunk looks back into the chunks before it.
-// With `claim`, a CTA takes its tile from an atomic counter instead of its blockIdx (see
-// tile_claim()).
+// The look-back relies on in-order dispatch of the blocks; a wait that nonetheless never ends gives
+// up after its poll limit with PARALLAX_ERR_DEVICE_SPIN. (A claim counter instead of blockIdx
+// measured 5-8 % slower.)
 template <typename T, bool EXCL, bool BULK, int NSUB>
 __global__ void __launch_bounds__(kBlock, kCtasPerSm)
 k_scan(const T* in, T* out, uint64_t n,  // in == out allowed (in-place ABI scan)
-       typename ScanTypes<T>::A init, TileStatus<typename ScanTypes<T>::A> ts, uint64_t tile0,
-       uint32_t* claim) {
+       typename ScanTypes<T>::A init, TileStatus<typename ScanTypes<T>::A> ts, uint64_t tile0) {
     using A = typename ScanTypes<T>::A;
     constexpr int SUB = ScanShape<T>::SUB;
     constexpr int TILE = NSUB * SUB;
@@ -206,10 +206,9 @@ k_scan(const T* in, T* out, uint64_t n,  // in == out allowed (in-place ABI scan
     __shared__ A s_tot[32];
     __shared__ A s_red[kBlock / 32 + 1];
     __shared__ int s_first[kBlock / 32];
-    __shared__ uint32_t s_claim;
     const int tid = threadIdx.x;
     dependent_prologue();
-    const uint64_t tile = tile0 + (claim ? tile_claim(claim, s_claim) : blockIdx.x);
+    const uint64_t tile = tile0 + blockIdx.x;
     const uint64_t base = tile * (uint64_t)TILE;
     const uint64_t rem = n - base;
     const uint32_t cnt = rem < (uint64_t)TILE ? (uint32_t)rem : (uint32_t)TILE;
@@ -221,7 +220,6 @@ k_scan(const T* in, T* out, uint64_t n,  // in == out allowed (in-place ABI scan
     if constexpr (BULK) {
         if (tid == 0 && bulk) bulk_wait_read_all();
     }
-    if (claim && tid == 0) persistent_exit(claim);
 }
 
 // Persistent pipeline without CTA-wide barriers. Operands 16-byte aligned.
@@ -425,12 +423,12 @@ k_scan_pipe(const T* in, T* out, uint64_t n, uint32_t num_tiles,
 template <typename T, bool EXCL, bool BULK, int NSUB = kSub>
 bool launch_tiles_single(const T* in, T* out, uint64_t n, typename ScanTypes<T>::A init,
                          TileStatus<typename ScanTypes<T>::A> ts, uint64_t count,
-                         cudaStream_t s, uint64_t tile0 = 0, uint32_t* claim = nullptr) {
+                         cudaStream_t s, uint64_t tile0 = 0) {
     constexpr size_t smem = (size_t)NSUB * ScanShape<T>::SUB * sizeof(T);
     if (!smem_opt_in<k_scan<T, EXCL, BULK, NSUB>>(smem))
         return cuda_ok(cudaGetLastError(), "k_scan shared-memory opt-in");
     return launch_dependent(k_scan<T, EXCL, BULK, NSUB>, (unsigned)count, kBlock, smem, s, "k_scan launch",
-                            in, out, n, init, ts, tile0, PXB_TILE_CLAIM ? claim : nullptr);
+                            in, out, n, init, ts, tile0);
 }
 
 template <typename T, bool EXCL>
@@ -454,14 +452,14 @@ template <typename T, bool EXCL>
 bool launch_scan_tiles(const T* in, T* out, uint64_t n, typename ScanTypes<T>::A init,
                        TileStatus<typename ScanTypes<T>::A> ts, uint64_t tiles, bool bulk,
                        uint32_t* counters, cudaStream_t s) {
-    if (!bulk) return launch_tiles_single<T, EXCL, false>(in, out, n, init, ts, tiles, s, 0, counters);
+    if (!bulk) return launch_tiles_single<T, EXCL, false>(in, out, n, init, ts, tiles, s);
     const uint64_t sms = device_info().sm_count;
     if (tiles <= sms / 2) {
         const uint64_t subs = (n + ScanShape<T>::SUB - 1) / ScanShape<T>::SUB;
-        return launch_tiles_single<T, EXCL, true, 1>(in, out, n, init, ts, subs, s, 0, counters);
+        return launch_tiles_single<T, EXCL, true, 1>(in, out, n, init, ts, subs, s);
     }
     if (tiles <= 2 * sms)
-        return launch_tiles_single<T, EXCL, true>(in, out, n, init, ts, tiles, s, 0, counters);
+        return launch_tiles_single<T, EXCL, true>(in, out, n, init, ts, tiles, s);
     return launch_pipe<T, EXCL>(in, out, n, init, ts, counters, s);
 }
 
@@ -567,10 +565,9 @@ bool scan_copies_typed(Workspace& ws, bool exclusive, const void* h_in, const vo
                 !cuda_ok(cudaStreamWaitEvent(s, ws.ev_copy[1], 0), "copy wait"))
                 return fail();
         }
-        uint32_t* counters = reinterpret_cast<uint32_t*>(scratch + ScratchOff::counters);
         const bool ok =
-            exclusive ? launch_tiles_single<T, true, true>(in, out, n, init, ts, t1 - t0, s, t0, counters)
-                      : launch_tiles_single<T, false, true>(in, out, n, init, ts, t1 - t0, s, t0, counters);
+            exclusive ? launch_tiles_single<T, true, true>(in, out, n, init, ts, t1 - t0, s, t0)
+                      : launch_tiles_single<T, false, true>(in, out, n, init, ts, t1 - t0, s, t0);
         if (!ok) return fail();
         if (h_out) {
             if (!cuda_ok(cudaEventRecord(ws.ev_copy[2], s), "copy event") ||

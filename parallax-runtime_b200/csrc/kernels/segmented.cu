@@ -25,9 +25,8 @@
 // are read element by element. Each thread then owns a row of VPT consecutive vectors; VPT
 // is odd, so the 16-byte row reads of a warp hit every bank once. Tiles hold
 // BLOCK x VPT vectors minus one (room for the phase shift).
-//   reduce     per-tile sum (max, min, or predicate count) -> per-item partial; the last
-//              tile of a segment to finish (per-segment ticket) folds the partials in item
-//              order (deterministic)
+//   reduce     per-tile sum (max, min, or predicate count) -> per-item partial; a pass of one
+//              warp per segment folds the partials in item order (deterministic)
 //   scan       row scans + warp shuffles + decoupled look-back that stops at the segment's
 //              first tile; results written back into the staged rows and stored with
 //              16-byte stores when the output has the input's phase
@@ -325,16 +324,11 @@ __device__ __forceinline__ uint32_t tile_ranks(uint32_t cnt, uint32_t* wcnt, uin
     return tot;
 }
 
-// Select / partition tiles walked warp-strided with one ballot per 32 elements
-// (PXB_SEG_STRIDED=1) instead of thread rows packed in shared memory (0). Measured on the
-// 4096-segment lognormal workload (122 M elements, x > 0.5 / x > 0): copy_if fp32 0.480 ms
-// strided against 0.550 ms in rows, int32 0.497 against 0.566 ms. (The same walk made the
+// Select / partition tiles are walked warp-strided with one ballot per 32 elements. Measured on
+// the 4096-segment lognormal workload (122 M elements, x > 0.5 / x > 0) against thread rows packed
+// in shared memory: copy_if fp32 0.480 / 0.550 ms, int32 0.497 / 0.566 ms. (The same walk made the
 // plain compaction kernels slower - copy_if 0.56 against 0.40 ms at 2^28 - whose rows read
 // their 112 KiB tiles with 16-byte loads and store packed runs; it is not used there.)
-#ifndef PXB_SEG_STRIDED
-#define PXB_SEG_STRIDED 1
-#endif
-
 __device__ __forceinline__ uint32_t lane_mask_lt() {
     uint32_t m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
@@ -522,19 +516,18 @@ k_segmented(SegArgs<T> a, SegBuffers b, volatile int32_t* err) {
             if (OP == SEG_SELECT && a.unique && tid == 0)
                 s_prev = begin > 0 ? in[begin - 1] : T(0);
             __syncthreads();
-            // this thread's row: slots [tid * ITEMS, +ITEMS) = tile indices from r0
-            [[maybe_unused]] const int r0 = tid * ITEMS - (int)mis;
-            T x[ITEMS];
-            {
-                const uint4* row = reinterpret_cast<const uint4*>(sm + tid * ITEMS);
-#pragma unroll
-                for (int v = 0; v < VPT; ++v) {
-                    const uint4 q = row[v];
-                    memcpy(&x[v * V], &q, 16);
-                }
-            }
             if constexpr (OP == SEG_SCAN) {
                 using L = typename SegRow<T>::type;
+                // this thread's row: slots [tid * ITEMS, +ITEMS)
+                T x[ITEMS];
+                {
+                    const uint4* row = reinterpret_cast<const uint4*>(sm + tid * ITEMS);
+    #pragma unroll
+                    for (int v = 0; v < VPT; ++v) {
+                        const uint4 q = row[v];
+                        memcpy(&x[v * V], &q, 16);
+                    }
+                }
                 L p[ITEMS];
                 p[0] = (L)x[0];
 #pragma unroll
@@ -575,7 +568,7 @@ k_segmented(SegArgs<T> a, SegBuffers b, volatile int32_t* err) {
                     for (uint32_t e = tid; e < len; e += BLOCK) out[begin + e] = sm[e + mis];
                 describe_next();
                 __syncthreads();
-            } else if constexpr (PXB_SEG_STRIDED) {  // SEG_SELECT / SEG_PARTITION, strided
+            } else {  // SEG_SELECT / SEG_PARTITION
                 // Warp w walks its slots [w * 32 * ITEMS, + 32 * ITEMS) 32 at a time: lane l
                 // holds slot w0 + 32 j + l (element slot - mis). One ballot per j ranks the
                 // kept lanes; each j's kept (and rejected) elements are one contiguous output
@@ -627,86 +620,6 @@ k_segmented(SegArgs<T> a, SegBuffers b, volatile int32_t* err) {
                 }
                 if (OP == SEG_SELECT && tid == 0 && k == it.seg_items - 1)
                     *reinterpret_cast<uint64_t*>(it.aux) = prefix + kept;
-                describe_next();
-                __syncthreads();
-            } else {  // SEG_SELECT / SEG_PARTITION
-                uint32_t f = 0;
-#pragma unroll
-                for (int j = 0; j < ITEMS; ++j) {
-                    const int i = r0 + j;
-                    bool keep;
-                    if (OP == SEG_SELECT && a.unique) {
-                        const T prev = i == 0 ? s_prev : j > 0 ? x[j - 1] : sm[tid * ITEMS - 1];
-                        keep = (begin == 0 && i == 0) || !(x[j] == prev);
-                    } else {
-                        keep = a.pred(x[j]);
-                    }
-                    if (i >= 0 && i < (int)len && keep) f |= 1u << j;
-                }
-                uint32_t kstart;
-                const uint32_t kept = tile_ranks<BLOCK>(__popc(f), wcnt, &kstart);
-                const uint64_t prefix =
-                    lookback_cta<uint64_t, BLOCK>(tsk, item, (uint64_t)kept, red64, first,
-                                                  it.first_item);
-                claim_next();
-                // Output warp by warp: warp w's rows are the staged slots [w * 32 * ITEMS,
-                // + 32 * ITEMS), whose kept elements form one contiguous output run (and, for
-                // partition, whose rejected ones form another), so each warp packs its own
-                // slots in place and stores its runs with no CTA-wide barrier.
-                T* const wsm = sm + warp * 32 * ITEMS;
-                {  // the row again, from shared memory (fewer registers live across the look-back)
-                    const uint4* row = reinterpret_cast<const uint4*>(sm + tid * ITEMS);
-#pragma unroll
-                    for (int v = 0; v < VPT; ++v) {
-                        const uint4 q = row[v];
-                        memcpy(&x[v * V], &q, 16);
-                    }
-                }
-                __syncwarp();  // every row of the warp is in registers before it is overwritten
-                const uint32_t wex = shfl_idx(kstart, 0);                      // kept before the warp
-                const uint32_t wk = shfl_idx(kstart + (uint32_t)__popc(f), 31) - wex;
-                uint32_t rk = kstart - wex;
-                if constexpr (OP == SEG_SELECT) {
-#pragma unroll
-                    for (int j = 0; j < ITEMS; ++j)
-                        if (f >> j & 1u) wsm[rk++] = x[j];
-                    __syncwarp();
-                    for (uint32_t i = lane; i < wk; i += 32) {
-                        if (prefix + wex + i < it.len) out[prefix + wex + i] = wsm[i];
-                        else *err = 3;
-                    }
-                    if (tid == 0 && k == it.seg_items - 1)
-                        *reinterpret_cast<uint64_t*>(it.aux) = prefix + kept;
-                } else {
-                    // rejected elements of the warp follow its kept run in its slots
-                    uint32_t valid = 0;
-#pragma unroll
-                    for (int j = 0; j < ITEMS; ++j) valid += (r0 + j >= 0 && r0 + j < (int)len);
-                    const uint32_t rej = valid - __popc(f);
-                    const uint32_t rincl = warp_inclusive_scan(rej, OpSum());
-                    const uint32_t wr = shfl_idx(rincl, 31);
-                    uint32_t rr = wk + rincl - rej;
-#pragma unroll
-                    for (int j = 0; j < ITEMS; ++j) {
-                        const int i = r0 + j;
-                        if (i < 0 || i >= (int)len) continue;
-                        if (f >> j & 1u) wsm[rk++] = x[j];
-                        else wsm[rr++] = x[j];
-                    }
-                    __syncwarp();
-                    // the segment's kept total, written by the count pass; the tile's rejected
-                    // elements start after the segment's kept run and the earlier tiles'
-                    // rejected ones, the warp's after the tile's earlier warps'
-                    const uint64_t seg_true = *reinterpret_cast<const uint64_t*>(it.aux);
-                    const int first_elem = warp * 32 * ITEMS - (int)mis;  // of the warp's slots
-                    const uint32_t before = first_elem <= 0 ? 0u : min((uint32_t)first_elem, len);
-                    const uint64_t rej_base = seg_true + (begin - prefix) + (before - wex);
-                    for (uint32_t i = lane; i < wk + wr; i += 32) {
-                        const uint64_t dst = i < wk ? prefix + wex + i : rej_base + (i - wk);
-                        if (dst < it.len) out[dst] = wsm[i];
-                        else *err = 3;
-                    }
-                }
                 describe_next();
                 __syncthreads();
             }
